@@ -49,7 +49,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-bool lbmx::encode_population_map(const lbmx_handle* h, CUtensorMap* out, int tile_w, int tile_h) {
+bool lbmx::encode_population_map(const lbmx_handle* h, CUtensorMap* out, int tile_w, int tile_h, void* f) {
     static EncodeTiledFn encode = nullptr;
     if (!encode) {
         void* fn = nullptr;
@@ -70,7 +70,7 @@ bool lbmx::encode_population_map(const lbmx_handle* h, CUtensorMap* out, int til
     const cuuint64_t strides[2] = {(cuuint64_t)h->g.pitch * es, (cuuint64_t)h->g.plane * es};
     const cuuint32_t box[3] = {(cuuint32_t)(tile_w + 2 * 16 / es), (cuuint32_t)tile_h, 1u};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
-    return encode(out, dt, 3, h->f, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    return encode(out, dt, 3, f ? f : h->f, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -115,16 +115,109 @@ StepArgs lbmx::base_args(const lbmx_handle* h) {
     return a;
 }
 
+// A device list in a buffer that only grows (a cudaFree / cudaMalloc pair per
+// list costs about as much as building it).
+static cudaError_t upload_list(const void* src, size_t bytes, void** buf, size_t* cap) {
+    if (!*buf || *cap < bytes) {
+        cudaFree(*buf);
+        *buf = nullptr;
+        *cap = 0;
+        const cudaError_t e = cudaMalloc(buf, std::max<size_t>(bytes, 4));
+        if (e != cudaSuccess) return e;
+        *cap = std::max<size_t>(bytes, 4);
+    }
+    return bytes ? cudaMemcpy(*buf, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
+}
+
+// General-path nodes of every two-step tile, from the unit lists of the two
+// steps: in the first step the tile's own and those of the ring of nodes
+// around it (across a periodic edge, the ring's node is the one on the other
+// side), in the second the tile's own.  Tiles with such nodes are claimed
+// first: they take longest.  Not paired: lattices whose steps need another
+// launch or exchange between them, and those with regularized boundaries,
+// whose arithmetic the compiler contracts differently in the two kernels (a
+// pair would differ from two single steps in the last bit).
+// Nor those with general-path nodes inside the domain beyond 1 in 128: in a
+// pair they are two passes in a row within their tile (and the ring's, again),
+// in a single step a chunk of their own (1024^2 FP32 with 2 % obstacle nodes:
+// 18.0 us a step in pairs, 14.0 in single steps).
+static lbmx_status rebuild_pair_lists(lbmx_handle* h, const std::vector<int>& units, const std::vector<int>& units0,
+                                      size_t inner_units) {
+    const Geometry& g = h->g;
+    if (2 * 128 * inner_units > (size_t)g.nx * g.ny) return LBMX_OK;
+    if (!h->f2 || h->p.op == LBMX_CM_OPT || (h->p.quirks & LBMX_QUIRK_REST_LAG) || h->ghost_mask || h->whole_ny > 0 ||
+        h->has_aux_bc || h->has_regularized || !h->patch_host.empty())
+        return LBMX_OK;
+    const int w = pair_w(h->pair_shape), hh = pair_h(h->pair_shape, (int)elem_size(h->p.storage));
+    const int tx = (g.nx + w - 1) / w, ty = (g.ny + hh - 1) / hh, nt = tx * ty;
+    // tiles (index along one axis) whose ring or interior holds coordinate v, and its place in them
+    struct Spot { int tile, d; };
+    const auto spots = [](int v, int n, int w, int tiles, bool periodic, bool ring, Spot out[4]) {
+        int k = 0;
+        out[k++] = Spot{v / w, v % w};
+        if (!ring) return k;
+        if (v > 0 && v % w == 0) out[k++] = Spot{v / w - 1, w};
+        if (v < n - 1 && v % w == w - 1) out[k++] = Spot{v / w + 1, -1};
+        if (periodic && v == 0) out[k++] = Spot{tiles - 1, n - (tiles - 1) * w};
+        if (periodic && v == n - 1) out[k++] = Spot{0, -1};
+        return k;
+    };
+    std::vector<int> at[2];
+    std::vector<std::pair<int, int>> found[2];  // {tile, entry}
+    for (int step = 0; step < 2; step++) {
+        for (int u : step ? units0 : units) {
+            const int y = u / g.pitch, x0 = u % g.pitch;
+            Spot sy[4], sx[4];
+            const int ky = spots(y, g.ny, hh, ty, g.periodic_y, step == 0, sy);
+            for (int x = x0; x < std::min(x0 + 2, g.nx); x++) {
+                const int fl = h->flags_host.empty() ? 0 : h->flags_host[(size_t)y * g.pitch + x];
+                const int kx = spots(x, g.nx, w, tx, g.periodic_x, step == 0, sx);
+                for (int i = 0; i < ky; i++)
+                    for (int j = 0; j < kx; j++)
+                        found[step].push_back({sy[i].tile * tx + sx[j].tile, fl << 16 | (sy[i].d + 1) << 8 | (sx[j].d + 1)});
+            }
+        }
+        at[step].assign((size_t)nt + 1, 0);
+        for (const auto& e : found[step]) at[step][(size_t)e.first + 1]++;
+        for (int t = 0; t < nt; t++) at[step][(size_t)t + 1] += at[step][(size_t)t];
+    }
+    const size_t n1 = found[0].size(), n0 = found[1].size();
+    std::vector<int> all((size_t)nt + 2 * ((size_t)nt + 1) + n1 + n0);
+    int* order = all.data();
+    int* at1 = order + nt;
+    int* at0 = at1 + nt + 1;
+    int k = 0;
+    for (int pass = 0; pass < 2; pass++)
+        for (int t = 0; t < nt; t++)
+            if ((at[0][(size_t)t + 1] > at[0][(size_t)t]) == (pass == 0)) order[k++] = t;
+    memcpy(at1, at[0].data(), at[0].size() * sizeof(int));
+    memcpy(at0, at[1].data(), at[1].size() * sizeof(int));
+    int* sp = at0 + nt + 1;
+    for (int step = 0; step < 2; step++) {
+        std::vector<int> fill(at[step].begin(), at[step].end() - 1);
+        for (const auto& e : found[step]) sp[fill[(size_t)e.first]++] = e.second;
+        sp += found[step].size();
+    }
+    LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
+    LBMX_CUDA(h, upload_list(all.data(), all.size() * sizeof(int), (void**)&h->pair_lists, &h->cap_pair_lists));
+    h->pair_tiles = nt;
+    h->pair_tiles_x = tx;
+    h->pair_sp1 = (int)n1;
+    h->pair_ready = true;
+    return LBMX_OK;
+}
+
 // Split the lattice between the two kinds of step-kernel work items: units
 // (two x-neighbouring nodes, x0 even) on the perimeter or holding a flagged
 // node take the general path; the kernel finds perimeter units by position
 // and the others through a bit per unit.  IBM patch nodes stay in the tiles,
 // which add the IBM force when they hold one.
-static lbmx_status rebuild_special(lbmx_handle* h) {
+static lbmx_status rebuild_special(lbmx_handle* h, bool pair_lists = true) {
     const Geometry& g = h->g;
     const int units_per_row = g.pitch / 2;
     const uint8_t* F = h->flags_host.empty() ? nullptr : h->flags_host.data();  // pitched, zero past nx
     bool any_interior = false;
+    size_t inner_units = 0;  // general-path units off the perimeter
     std::vector<int> units, units0;
     std::vector<uint32_t> bits(((size_t)g.ny * units_per_row + 31) / 32, 0u), bits0(bits.size(), 0u);
     const auto set_bit = [](std::vector<uint32_t>& b, size_t u) { b[u >> 5] |= 1u << (u & 31); };
@@ -158,6 +251,7 @@ static lbmx_status rebuild_special(lbmx_handle* h) {
             const size_t u = u_row + x0 / 2;
             if (perim || flagged || wrap_row) units.push_back(y * g.pitch + x0);
             if (!perim && (flagged || wrap_row)) {
+                inner_units++;
                 set_bit(bits, u);
                 any_interior = true;
             }
@@ -220,31 +314,27 @@ static lbmx_status rebuild_special(lbmx_handle* h) {
         });
         return (int)(it - list.begin());
     };
+    // the two-step launches' lists: with the flags, or before the first pair
+    // of a lattice that never gets any
+    h->pair_ready = h->pair_stale = false;
+    if (!pair_lists) {
+        h->pair_stale = true;
+    } else {
+        const lbmx_status ps = rebuild_pair_lists(h, units, units0, inner_units);
+        if (ps != LBMX_OK) return ps;
+    }
     const int indep = by_patch(units), indep0 = by_patch(units0);
-    // device copies, in buffers that only grow (a cudaFree / cudaMalloc pair
-    // per list cost about as much as building the lists); null unit bits:
-    // none marked
+    // device copies; null unit bits: none marked
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
-    const auto upload = [&](const void* src, size_t bytes, void** buf, size_t* cap) -> cudaError_t {
-        if (!*buf || *cap < bytes) {
-            cudaFree(*buf);
-            *buf = nullptr;
-            *cap = 0;
-            const cudaError_t e = cudaMalloc(buf, std::max<size_t>(bytes, 4));
-            if (e != cudaSuccess) return e;
-            *cap = std::max<size_t>(bytes, 4);
-        }
-        return bytes ? cudaMemcpy(*buf, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
-    };
-    LBMX_CUDA(h, upload(units.data(), units.size() * sizeof(int), (void**)&h->special_units, &h->cap_units));
-    LBMX_CUDA(h, upload(units0.data(), units0.size() * sizeof(int), (void**)&h->special_units0, &h->cap_units0));
+    LBMX_CUDA(h, upload_list(units.data(), units.size() * sizeof(int), (void**)&h->special_units, &h->cap_units));
+    LBMX_CUDA(h, upload_list(units0.data(), units0.size() * sizeof(int), (void**)&h->special_units0, &h->cap_units0));
     h->special_bits = h->special_bits0 = nullptr;
     if (any_interior) {
-        LBMX_CUDA(h, upload(bits.data(), bits.size() * sizeof(uint32_t), (void**)&h->bits_buf, &h->cap_bits));
+        LBMX_CUDA(h, upload_list(bits.data(), bits.size() * sizeof(uint32_t), (void**)&h->bits_buf, &h->cap_bits));
         h->special_bits = h->bits_buf;
     }
     if (!units0.empty() || h->ghost_mask) {
-        LBMX_CUDA(h, upload(bits0.data(), bits0.size() * sizeof(uint32_t), (void**)&h->bits0_buf, &h->cap_bits0));
+        LBMX_CUDA(h, upload_list(bits0.data(), bits0.size() * sizeof(uint32_t), (void**)&h->bits0_buf, &h->cap_bits0));
         h->special_bits0 = h->bits0_buf;
     }
     h->nspecial = (int)units.size();
@@ -303,12 +393,6 @@ static lbmx_status rebuild_special(lbmx_handle* h) {
     };
     split(h->special_chunks, &h->num_ctas, &h->tile_chunk);
     split(h->special_chunks0, &h->num_ctas0, &h->tile_chunk0);
-    if (!h->partials) {
-        // two sets (one per step parity) of kSumSlots copies of the six
-        // fixed-point grid accumulators (zero between uses)
-        LBMX_CUDA(h, cudaMalloc((void**)&h->partials, (size_t)2 * kAccPerSet * sizeof(double)));
-        LBMX_CUDA(h, cudaMemset(h->partials, 0, (size_t)2 * kAccPerSet * sizeof(double)));
-    }
     return LBMX_OK;
 }
 
@@ -354,6 +438,15 @@ void lbmx::set_step(const lbmx_handle* h, StepArgs& a, long long s) {
                                 : (long long)opp[q] * g.plane) * es;
 }
 
+// The two edge stores alike: a pair writes the values its steps produce into
+// the other one, and the rest (nodes that are half-way walls for now) must be
+// there already.
+static cudaError_t copy_edge(lbmx_handle* h) {
+    if (!h->edge2) return cudaSuccess;
+    return cudaMemcpyAsync(h->edge2, h->edge, (size_t)2 * h->g.perimeter * 9 * sizeof(float), cudaMemcpyDeviceToDevice,
+                           h->stream);
+}
+
 static void free_ibm(lbmx_handle* h) {
     cudaFree(h->patch_nodes); cudaFree(h->sten_idx); cudaFree(h->sten_w); cudaFree(h->spread);
     cudaFree(h->marker_u);
@@ -387,12 +480,11 @@ void lbmx_destroy(lbmx_handle* h) {
     cudaSetDevice(h->p.device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     free_ibm(h);
-    cudaFree(h->f_alloc); cudaFree(h->flags); cudaFree(h->edge); cudaFree(h->aux);
-    cudaFree(h->force); cudaFree(h->gamma); cudaFree(h->rho_out); cudaFree(h->u_out); cudaFree(h->staging);
-    cudaFree(h->pop_out); cudaFree(h->partials); cudaFree(h->counter); cudaFree(h->sums); cudaFree(h->raw_sums);
-    cudaFree(h->avg); cudaFree(h->error_word); cudaFree(h->special_units); cudaFree(h->bits_buf);
-    cudaFree(h->special_units0); cudaFree(h->bits0_buf); cudaFree(h->tile_order);
-    cudaFree(h->tile_counter);
+    if (h->staging != h->f2) cudaFree(h->staging);
+    cudaFree(h->f_alloc); cudaFree(h->edge_alloc); cudaFree(h->words); cudaFree(h->pair_lists); cudaFree(h->flags);
+    cudaFree(h->force); cudaFree(h->gamma); cudaFree(h->rho_out); cudaFree(h->pop_out); cudaFree(h->raw_sums);
+    cudaFree(h->special_units); cudaFree(h->bits_buf); cudaFree(h->special_units0); cudaFree(h->bits0_buf);
+    cudaFree(h->tile_order);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
     cudaSetDevice(cur);
     delete h;
@@ -441,26 +533,58 @@ lbmx_status lbmx_create(const lbmx_params* p, lbmx_handle** out) {
             return LBMX_ERR_OUT_OF_MEMORY;                                                  \
         }                                                                                   \
     } while (0)
-    ALLOC(h->f_alloc, ((size_t)h->nplanes * g.plane + 2 * kGuardElems) * elem_size(p->storage));
-    h->f = static_cast<char*>(h->f_alloc) + (size_t)kGuardElems * elem_size(p->storage);
     cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, p->device);
     if (h->num_sms < 1) h->num_sms = 1;
-    if (!encode_population_map(h, &h->tmap, step_tile_w((int)elem_size(p->storage)),
-                               step_tile_h((int)elem_size(p->storage)))) {
+    // The populations, and the second population buffer of the two-step
+    // launches while the device keeps at least half of its memory free beside
+    // it (a spare that lattices created later may need instead).  It holds
+    // the init fields too: nothing else is in it between launches.
+    const int es = (int)elem_size(p->storage);
+    const size_t f_bytes = (((size_t)h->nplanes * g.plane + 2 * kGuardElems) * es + 255) / 256 * 256;
+    size_t free_b = 0, total_b = 0;
+    const bool pairs = p->op != LBMX_CM_OPT && !(p->quirks & LBMX_QUIRK_REST_LAG) &&
+                       (unsigned long long)g.plane * es <= 0xFFFFFFFFull &&
+                       cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b >= 2 * f_bytes + total_b / 2 &&
+                       cudaMalloc(&h->f_alloc, 2 * f_bytes) == cudaSuccess;
+    if (!pairs) {
+        cudaGetLastError();
+        ALLOC(h->f_alloc, f_bytes);
+    }
+    h->f = static_cast<char*>(h->f_alloc) + (size_t)kGuardElems * es;
+    if (pairs) h->f2 = static_cast<char*>(h->f) + f_bytes;
+    h->pair_shape = pair_shape(g.nx, g.ny, es, p->op, h->num_sms);
+    const int tw = step_tile_w(es), th = step_tile_h(es), pw = pair_w(h->pair_shape), ph = pair_h(h->pair_shape, es) + 2;
+    bool maps = encode_population_map(h, &h->tmap, tw, th);
+    if (pairs)
+        maps = maps && encode_population_map(h, &h->tmap2, tw, th, h->f2) &&
+               encode_population_map(h, &h->pair_tmap[0], pw, ph) &&
+               encode_population_map(h, &h->pair_tmap[1], pw, ph, h->f2);
+    if (!maps) {
         fail(nullptr, LBMX_ERR_CUDA, "lbmx_create: cannot build the TMA descriptor (cuTensorMapEncodeTiled)");
         lbmx_destroy(h);
         return LBMX_ERR_CUDA;
     }
-    ALLOC(h->edge, (size_t)2 * g.perimeter * 9 * sizeof(float));
-    ALLOC(h->aux, (size_t)g.perimeter * 9 * sizeof(float));
-    ALLOC(h->rho_out, (size_t)g.plane * sizeof(float));
-    ALLOC(h->u_out, (size_t)2 * g.plane * sizeof(float));
-    ALLOC(h->staging, (size_t)3 * n * sizeof(float));
-    ALLOC(h->counter, sizeof(unsigned int));
-    ALLOC(h->sums, kSumsBufferLen * sizeof(double));
-    ALLOC(h->avg, 3 * sizeof(float));
-    ALLOC(h->error_word, sizeof(unsigned int));
-    ALLOC(h->tile_counter, 2 * sizeof(unsigned long long));
+    // the edge store(s) and the edge pre-pass' neighbour data
+    const size_t edge_n = (size_t)g.perimeter * 9;
+    ALLOC(h->edge_alloc, (pairs ? 5 : 3) * edge_n * sizeof(float));
+    h->aux = h->edge_alloc;
+    h->edge = h->aux + edge_n;
+    h->edge2 = pairs ? h->edge + 2 * edge_n : nullptr;
+    ALLOC(h->rho_out, (size_t)3 * g.plane * sizeof(float));
+    h->u_out = h->rho_out + g.plane;
+    if (h->f2) h->staging = static_cast<float*>(h->f2);
+    else ALLOC(h->staging, (size_t)3 * n * sizeof(float));
+    // the small device words in one allocation, zeroed: the grid accumulators
+    // (kAccSets sets of kSumSlots copies, zero between uses), the sums, the
+    // work counters, the averages, the last-block counter and the error word
+    const size_t words = (size_t)(kAccSets * kAccPerSet + kSumsBufferLen + 4) * 8 + 5 * 4;
+    ALLOC(h->words, words);
+    h->partials = static_cast<double*>(h->words);
+    h->sums = h->partials + kAccSets * kAccPerSet;
+    h->tile_counter = reinterpret_cast<unsigned long long*>(h->sums + kSumsBufferLen);
+    h->avg = reinterpret_cast<float*>(h->tile_counter + 4);
+    h->counter = reinterpret_cast<unsigned int*>(h->avg + 3);
+    h->error_word = h->counter + 1;
 #undef ALLOC
     if (p->stream) {
         h->stream = (cudaStream_t)p->stream;
@@ -472,18 +596,14 @@ lbmx_status lbmx_create(const lbmx_params* p, lbmx_handle** out) {
         }
         h->own_stream = true;
     }
-    cudaMemsetAsync(h->counter, 0, sizeof(unsigned int), h->stream);
-    cudaMemsetAsync(h->sums, 0, kSumsBufferLen * sizeof(double), h->stream);
-    cudaMemsetAsync(h->avg, 0, 3 * sizeof(float), h->stream);
-    cudaMemsetAsync(h->error_word, 0, sizeof(unsigned int), h->stream);
-    cudaMemsetAsync(h->tile_counter, 0, 2 * sizeof(unsigned long long), h->stream);
+    cudaMemsetAsync(h->words, 0, words, h->stream);
     cudaMemsetAsync(h->aux, 0, (size_t)g.perimeter * 9 * sizeof(float), h->stream);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
         fail(nullptr, LBMX_ERR_CUDA, "lbmx_create: initial clears failed");
         lbmx_destroy(h);
         return LBMX_ERR_CUDA;
     }
-    if (rebuild_special(h) != LBMX_OK) {
+    if (rebuild_special(h, false) != LBMX_OK) {
         fail(nullptr, LBMX_ERR_OUT_OF_MEMORY, "lbmx_create: %s", h->err);
         lbmx_destroy(h);
         return LBMX_ERR_OUT_OF_MEMORY;
@@ -510,7 +630,7 @@ lbmx_status lbmx_set_flags(lbmx_handle* h, const uint8_t* flags) {
         cudaGetLastError();
         LBMX_CUDA(h, cudaMemcpy(hf.data(), flags, n, cudaMemcpyDefault));
     }
-    bool any = false, aux = false;
+    bool any = false, aux = false, reg = false;
     for (int y = 0; y < g.ny; y++)
         for (int x = 0; x < g.nx; x++) {
             const uint8_t* r = &hf[(long long)y * g.nx];
@@ -537,12 +657,14 @@ lbmx_status lbmx_set_flags(lbmx_handle* h, const uint8_t* flags) {
                             "lbmx_set_flags: PRESSURE_OUTLET at (%d,%d) must sit on the domain edge with x >= 1", x, y);
             if ((fl == LBMX_ZG_OUTFLOW || fl == LBMX_REGULARIZED_BOUNCE_BACK_CORNER) && edge) aux = true;
             if (fl == LBMX_PRESSURE_OUTLET) aux = true;
+            if (fl == LBMX_REGULARIZED_INLET_TOP || fl == LBMX_REGULARIZED_BOUNCE_BACK) reg = true;
         }
+    LBMX_CUDA(h, copy_edge(h));
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
     if (!any) {
         cudaFree(h->flags);
         h->flags = nullptr;
-        h->has_aux_bc = false;
+        h->has_aux_bc = h->has_regularized = false;
         h->flags_host.clear();
         return rebuild_special(h);
     }
@@ -555,6 +677,7 @@ lbmx_status lbmx_set_flags(lbmx_handle* h, const uint8_t* flags) {
         memcpy(&h->flags_host[(size_t)y * g.pitch], &hf[(size_t)y * g.nx], g.nx);
     LBMX_CUDA(h, cudaMemcpy(h->flags, h->flags_host.data(), (size_t)g.plane, cudaMemcpyHostToDevice));
     h->has_aux_bc = aux;
+    h->has_regularized = reg;
     return rebuild_special(h);
 }
 
@@ -639,14 +762,17 @@ lbmx_status lbmx_init_from_fields(lbmx_handle* h, const float* rho, const float*
     LBMX_CUDA(h, dispatch(h->p.storage, [&](auto tag) {
                   return launch_init<decltype(tag)>(a, h->staging, h->staging + n, h->stream);
               }));
+    LBMX_CUDA(h, copy_edge(h));
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
     h->t = 0;
     h->last_step = -2;
-    h->pend_acc = h->pend_series = nullptr;
+    h->pend_acc = h->pend_series = h->pend_acc2 = h->pend_series2 = nullptr;
     h->initialized = true;
     h->have_avg = false;
     return LBMX_OK;
 }
+
+static lbmx_status flush_sums(lbmx_handle* h);
 
 // One step (index s = t+1); store: write moments and FP64 sums; sums: the
 // FP64 sums only; ke: the sums include the kinetic energy; series: where the
@@ -661,7 +787,7 @@ static lbmx_status run_step(lbmx_handle* h, bool store, bool check, bool sums, b
     // this step's work counter was zeroed by the previous launch, unless that
     // was not this handle's previous step (a fresh state, batched steps)
     if (h->last_step != s - 1)
-        LBMX_CUDA(h, cudaMemsetAsync(h->tile_counter, 0, 2 * sizeof(unsigned long long), st));
+        LBMX_CUDA(h, cudaMemsetAsync(h->tile_counter, 0, 4 * sizeof(unsigned long long), st));
     double* acc = h->partials + (size_t)(s & 1) * kAccPerSet;
     if (h->has_aux_bc)
         LBMX_CUDA(h, dispatch(storage, [&](auto tag) { return launch_edge_prepass<decltype(tag)>(a, h->aux, st); }));
@@ -717,12 +843,17 @@ static lbmx_status run_step(lbmx_handle* h, bool store, bool check, bool sums, b
     // with the IBM kernel just launched, the step starts on the items away
     // from the patch while the marker rounds run
     a.early = h->nm > 0 ? 1 : 0;
-    // the previous step's sums, if it left them to this launch
+    // the previous step's sums, if it left them to this launch (a pair's two
+    // are published by themselves)
+    if (h->pend_acc2) {
+        const lbmx_status fs = flush_sums(h);
+        if (fs != LBMX_OK) return fs;
+    }
     if (h->pend_acc) {
         a.pub_acc = h->pend_acc;
         a.pub_sums = h->sums;
         a.pub_series = h->pend_series;
-        h->pend_acc = h->pend_series = nullptr;
+        h->pend_acc = h->pend_series = h->pend_acc2 = h->pend_series2 = nullptr;
     }
     LBMX_CUDA(h, dispatch(storage, [&](auto tag) { return launch_step<decltype(tag)>(a, h->tmap, h->p.op, st); }));
     if (step_mode(a) == kModeSums) {
@@ -734,11 +865,108 @@ static lbmx_status run_step(lbmx_handle* h, bool store, bool check, bool sums, b
     return LBMX_OK;
 }
 
+// Two steps (indices s = t+1, odd, and t+2) in one launch; store, check and
+// series2 belong to the second, sums and ke to both.
+static lbmx_status run_pair(lbmx_handle* h, bool store, bool check, bool sums, bool ke, double* series1 = nullptr,
+                            double* series2 = nullptr) {
+    const long long s = h->t + 1;
+    PairArgs p;
+    memset(&p, 0, sizeof(p));
+    p.a = base_args(h);
+    set_step(h, p.a, s);
+    p.b = base_args(h);
+    set_step(h, p.b, s + 1);
+    p.b.f = h->f2;
+    p.b.edge = h->edge2;
+    p.edge_in = h->edge;
+    p.ntiles = h->pair_tiles;
+    p.tiles_x = h->pair_tiles_x;
+    p.shape = h->pair_shape;
+    p.num_sms = h->num_sms;
+    p.order = h->pair_lists;
+    p.sp1_at = p.order + p.ntiles;
+    p.sp0_at = p.sp1_at + p.ntiles + 1;
+    p.sp1 = p.sp0_at + p.ntiles + 1;
+    p.sp0 = p.sp1 + h->pair_sp1;
+    // each pair's launch zeroes the next one's counter and the single steps'
+    if (h->last_step != s - 1)
+        LBMX_CUDA(h, cudaMemsetAsync(h->tile_counter, 0, 4 * sizeof(unsigned long long), h->stream));
+    p.step_counters = h->tile_counter;
+    p.counter = h->tile_counter + 2 + (h->pair_seq & 1);
+    p.counter_next = h->tile_counter + 2 + ((h->pair_seq + 1) & 1);
+    double* acc = h->partials + (size_t)(2 + 2 * (h->pair_seq & 1)) * kAccPerSet;
+    p.b.counter = h->counter;
+    if (sums) {
+        p.a.partials = acc;
+        p.a.sums = h->sums;
+        p.a.ke = ke ? 1 : 0;
+        p.a.series = series1;
+    }
+    if (sums || store) {
+        p.b.partials = acc + kAccPerSet;
+        p.b.sums = h->sums;
+        p.b.ke = ke ? 1 : 0;
+        p.b.series = series2;
+    }
+    if (store) {
+        p.b.rho_out = h->rho_out;
+        p.b.u_out = h->u_out;
+    }
+    p.b.check_finite = check ? 1 : 0;
+    if (h->pend_acc) {
+        p.a.pub_acc = h->pend_acc;
+        p.a.pub_sums = h->sums;
+        p.a.pub_series = h->pend_series;
+        p.pub_acc2 = h->pend_acc2;
+        p.pub_series2 = h->pend_series2;
+        h->pend_acc = h->pend_series = h->pend_acc2 = h->pend_series2 = nullptr;
+    }
+    LBMX_CUDA(h, dispatch(h->p.storage, [&](auto tag) {
+                  return launch_pair<decltype(tag)>(p, h->pair_tmap[0], h->p.op, h->stream);
+              }));
+    if (pair_mode(p) == kModeSums) {
+        // (its first step's too, if it has any)
+        h->pend_acc = sums ? acc : acc + kAccPerSet;
+        h->pend_series = sums ? series1 : series2;
+        h->pend_acc2 = sums ? acc + kAccPerSet : nullptr;
+        h->pend_series2 = sums ? series2 : nullptr;
+    }
+    // the state is in the other buffers now
+    std::swap(h->f, h->f2);
+    std::swap(h->edge, h->edge2);
+    std::swap(h->tmap, h->tmap2);
+    std::swap(h->pair_tmap[0], h->pair_tmap[1]);
+    h->staging = static_cast<float*>(h->f2);
+    h->pair_seq++;
+    h->last_step = s + 1;
+    h->t = s + 1;
+    return LBMX_OK;
+}
+
+// Whether this call's steps may go in pairs: not into a capture, whose
+// replays would start from the buffer the state was in when it was captured.
+// Large 16-bit lattices, where both kernels are bound by instruction issue,
+// keep to single steps when every step reduces sums, which a pair reduces
+// with less occupancy (4096^2 FP16 BGK with sums 126 us a step, 130 in
+// pairs; with the kinetic energy 160 and 183; without sums 111 and 108).
+static bool can_pair(lbmx_handle* h, bool every_step_sums) {
+    if (!(h->pair_ready || h->pair_stale) || h->in_batch || h->nm > 0) return false;
+    if (every_step_sums && h->pair_shape == 0 && elem_size(h->p.storage) == 2) return false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (cs != cudaStreamCaptureStatusNone) return false;
+    return !h->pair_stale || (rebuild_special(h) == LBMX_OK && h->pair_ready);
+}
+
 // Publish sums a step left to the next launch when no step follows.
 static lbmx_status flush_sums(lbmx_handle* h) {
     if (!h->pend_acc) return LBMX_OK;
     LBMX_CUDA(h, launch_publish(h->pend_acc, h->sums, h->pend_series, h->stream));
-    h->pend_acc = h->pend_series = nullptr;
+    if (h->pend_acc2) LBMX_CUDA(h, launch_publish(h->pend_acc2, h->sums, h->pend_series2, h->stream));
+    h->pend_acc = h->pend_series = h->pend_acc2 = h->pend_series2 = nullptr;
     return LBMX_OK;
 }
 
@@ -750,11 +978,14 @@ lbmx_status lbmx_step_ex(lbmx_handle* h, int32_t nsteps, uint32_t flags) {
     const bool check = (flags & LBMX_STEP_CHECK_FINITE) != 0;
     if (check) LBMX_CUDA(h, cudaMemsetAsync(h->error_word, 0, sizeof(unsigned int), h->stream));
     const bool ke = (flags & LBMX_STEP_KINETIC_ENERGY) != 0;
-    for (int i = 0; i < nsteps; i++) {
-        const bool last = i == nsteps - 1;
-        lbmx_status st = run_step(h, last && (flags & LBMX_STEP_STORE_MOMENTS), last && check,
-                                  (flags & LBMX_STEP_SUMS) != 0, ke);
+    const bool pairs = can_pair(h, (flags & LBMX_STEP_SUMS) != 0);
+    for (int i = 0; i < nsteps;) {
+        const int k = pairs && !(h->t & 1) && nsteps - i >= 2 ? 2 : 1;
+        const bool last = i + k == nsteps;
+        const bool store = last && (flags & LBMX_STEP_STORE_MOMENTS), sums = (flags & LBMX_STEP_SUMS) != 0;
+        const lbmx_status st = k == 2 ? run_pair(h, store, last && check, sums, ke) : run_step(h, store, last && check, sums, ke);
         if (st != LBMX_OK) return st;
+        i += k;
     }
     lbmx_status fs = flush_sums(h);
     if (fs != LBMX_OK) return fs;
@@ -788,7 +1019,16 @@ lbmx_status lbmx_step_sums(lbmx_handle* h, int32_t nsteps, uint32_t flags, doubl
     // a step's entry: {rho, rho ux, rho uy}, then the kinetic energy
     const bool ke = (flags & LBMX_STEP_KINETIC_ENERGY) != 0;
     const size_t stride = ke ? 4 : 3;
+    const bool pairs = direct && can_pair(h, true);
     for (int i = 0; i < nsteps; i++) {
+        if (pairs && !(h->t & 1) && nsteps - i >= 2) {
+            const bool ends = i + 2 == nsteps;
+            const lbmx_status st = run_pair(h, ends && (flags & LBMX_STEP_STORE_MOMENTS), ends && check, true, ke,
+                                            dev_series + stride * (size_t)i, dev_series + stride * (size_t)(i + 1));
+            if (st != LBMX_OK) return st;
+            i++;
+            continue;
+        }
         const bool last = i == nsteps - 1;
         lbmx_status st = run_step(h, last && (flags & LBMX_STEP_STORE_MOMENTS), last && check, true, ke,
                                   direct ? dev_series + stride * (size_t)i : nullptr);
@@ -1258,9 +1498,11 @@ lbmx_status lbmx_checkpoint_load(lbmx_handle* h, const char* path) {
     LBMX_CUDA(h, cudaMemcpy(h->f, f.data(), f.size(), cudaMemcpyHostToDevice));
     LBMX_CUDA(h, cudaMemcpy(h->edge, edge.data(), edge.size(), cudaMemcpyHostToDevice));
     LBMX_CUDA(h, cudaMemcpy(h->avg, avg, sizeof(avg), cudaMemcpyHostToDevice));
+    LBMX_CUDA(h, copy_edge(h));
+    LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
     h->t = hd.t;
     h->last_step = -2;
-    h->pend_acc = h->pend_series = nullptr;
+    h->pend_acc = h->pend_series = h->pend_acc2 = h->pend_series2 = nullptr;
     h->initialized = true;
     h->have_avg = h->p.op == LBMX_CM_OPT && hd.t > 0;
     return LBMX_OK;

@@ -374,6 +374,7 @@ lbmx_status lbmx_batch_create(lbmx_handle* const* lattices, int32_t count, lbmx_
     cudaMemsetAsync(b->done, 0, sizeof(unsigned int), b->stream);
     cudaMemsetAsync(b->error_word, 0, sizeof(unsigned int), b->stream);
     if (refresh(b) != LBMX_OK) return cleanup(LBMX_ERR_CUDA, b->err);
+    for (lbmx_handle* h : b->lat) h->in_batch = true;
     *out = b;
     return LBMX_OK;
 }

@@ -18,6 +18,7 @@ struct lbmx_handle {
     int nplanes = 9;
     uint8_t* flags = nullptr;      // device, pitched; null while every node is fluid
     bool has_aux_bc = false;
+    bool has_regularized = false;  // a regularized inlet or wall
     float* edge = nullptr;         // [2][perimeter][9]
     float* aux = nullptr;          // [perimeter][9]
     float* force = nullptr;        // [2][plane] optional per-node body force
@@ -27,7 +28,7 @@ struct lbmx_handle {
     float* u_out = nullptr;        // [2][plane]
     float* staging = nullptr;      // dense [3][n] upload / readback staging
     float* pop_out = nullptr;      // dense [9][n] readback staging
-    double* partials = nullptr;    // [2][kAccPerSet] fixed-point grid accumulators of the step's sums
+    double* partials = nullptr;    // [kAccSets][kAccPerSet] fixed-point grid accumulators of the steps' sums
     unsigned int* counter = nullptr;
     double* sums = nullptr;        // [6]
     float* avg = nullptr;          // [3]
@@ -68,11 +69,32 @@ struct lbmx_handle {
     int* tile_order = nullptr;          // tiles away from the IBM patch, then the others (null without markers)
     int dep_tile = 0;                   // tiles away from the patch
     int nspecial = 0, special_chunks = 0, tiles_x = 0, tiles_y = 0, num_ctas = 0, num_sms = 1;
-    void* f_alloc = nullptr;  // population allocation including the guard elements
-    unsigned long long* tile_counter = nullptr;  // [2] work counters, alternating by step
+    void* f_alloc = nullptr;  // population allocation (f and f2) including the guard elements
+    float* edge_alloc = nullptr;  // aux, edge and edge2
+    void* words = nullptr;        // partials, sums, counters, averages, error word
+    // [4] work counters: two of the single-step kernel, alternating by step,
+    // and two of the two-step kernel, alternating by pair
+    unsigned long long* tile_counter = nullptr;
+    // Two-step launches (lbmx_pair_kernels.cuh): the second population buffer
+    // and edge store, which a pair writes and then swaps with f and edge;
+    // null where there is no room for them (every step is then a single one)
+    void* f2 = nullptr;
+    float* edge2 = nullptr;
+    CUtensorMap tmap2;                // f2's descriptor for the single-step tiles
+    CUtensorMap pair_tmap[2];         // descriptors of f and f2 for the two-step tiles
+    int* pair_lists = nullptr;        // order, sp1_at, sp0_at, sp1, sp0 (PairArgs) in one buffer
+    size_t cap_pair_lists = 0;
+    int pair_tiles = 0, pair_tiles_x = 0, pair_sp1 = 0;  // tiles, tiles per row, entries of sp1
+    int pair_shape = 0;               // tile shape (lbmx::pair_w, pair_h)
+    bool pair_stale = false;          // the lists are still to be built
+    bool pair_ready = false;          // the lists match the flags and the lattice's steps can be paired
+    bool in_batch = false;            // a batch keeps this lattice's buffer addresses: single steps only
+    unsigned long long pair_seq = 0;  // pairs launched
     long long last_step = -2;      // step index of the last single-lattice launch
     double* pend_acc = nullptr;    // accumulators of a step whose sums are not yet published
     double* pend_series = nullptr; // and that step's series entry or null
+    double* pend_acc2 = nullptr;   // after a pair: its second step's accumulators and entry
+    double* pend_series2 = nullptr;
     int tile_chunk = 1;            // neighbour-access steps (num_ctas, tile_chunk) and own-node
     int num_ctas0 = 0, tile_chunk0 = 1;  // steps (num_ctas0, tile_chunk0)
     CUtensorMap tmap;  // the type carries the 64-byte alignment TMA needs  // TMA descriptor of the population planes
@@ -88,7 +110,8 @@ StepArgs base_args(const lbmx_handle* h);
 // parity and rest-population plane of step index s (1-based)
 void set_step(const lbmx_handle* h, StepArgs& a, long long s);
 // 3-D tiled TMA descriptor over the population planes for tile_w x tile_h tiles
-bool encode_population_map(const lbmx_handle* h, CUtensorMap* out, int tile_w, int tile_h);
+// (of the buffer f, by default the handle's current one)
+bool encode_population_map(const lbmx_handle* h, CUtensorMap* out, int tile_w, int tile_h, void* f = nullptr);
 // Peskin stencils of n markers (host array xy[2k], xy[2k+1]) on an nx x ny
 // lattice with row pitch `pitch`: sidx / sw [n][S*S] (S = 2 or 4) patch index
 // (-1 outside the lattice) and weight, nodes the patch's node offsets.

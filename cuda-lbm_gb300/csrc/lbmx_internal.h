@@ -4,6 +4,8 @@
 #include <cuda.h>  // CUtensorMap (the descriptor type only; no driver calls are linked)
 #include <cuda_runtime.h>
 
+#include "lbmx.h"
+
 namespace lbmx {
 
 // Geometry and storage of one lattice in HBM.
@@ -113,6 +115,32 @@ __host__ __device__ inline int edge_index(int x, int y, int nx, int ny) {
     return 2 * nx + (ny - 2) + (y - 1);
 }
 
+// Two steps in one launch (lbmx_pair_kernels.cuh).
+struct PairArgs {
+    StepArgs a;                // the neighbour-access step; a.f and a.edge are read only
+    StepArgs b;                // the own-node step after it; b.f and b.edge are the buffers written
+    const float* edge_in;      // a.edge again: the own-node step's old edge-store values
+    const int* order;          // [ntiles] tiles in claim order
+    int ntiles, tiles_x;
+    int shape;                 // tile shape (pair_w, pair_h)
+    int num_sms;
+    // general-path nodes of each tile t, entries sp[sp_at[t]] .. sp[sp_at[t + 1]]:
+    // {flag, dy + 1, dx + 1} in bytes 2, 1 and 0, (dx, dy) from the tile's first node
+    const int* sp1_at;         // first step: the tile's nodes and the ring around it
+    const int* sp1;
+    const int* sp0_at;         // second step: the tile's nodes
+    const int* sp0;
+    unsigned long long* counter;        // next tile to claim (this launch's of two)
+    unsigned long long* counter_next;   // zeroed for the next pair
+    unsigned long long* step_counters;  // [2] the single-step kernel's, zeroed too
+    // a pair before this one left its second step's sums too: published
+    // after its first's (a.pub_acc)
+    double* pub_acc2;
+    double* pub_series2;
+};
+template <typename T>
+cudaError_t launch_pair(const PairArgs& p, const CUtensorMap& tmap, int op, cudaStream_t s);
+
 // host launchers (one translation unit per storage type)
 // tmap: 3-D tiled TMA descriptor over the population planes,
 // dims {pitch, ny, planes}, box {kStageW + 2 * 16 B of halo, kStageH, 1}
@@ -187,6 +215,9 @@ constexpr int kNumSums = 6;
 constexpr int kSumKE = 3;
 constexpr int kSumSlots = 32;
 constexpr int kAccPerSet = kSumSlots * kNumSums;
+// sets of a handle: one per step parity for single steps, two for each of
+// two alternating pairs
+constexpr int kAccSets = 6;
 // the handle's sums buffer holds two more doubles after the sums: the
 // drag / lift slot lbmx_step_forces copies pageable series from
 constexpr int kSumForces = kNumSums;
@@ -202,12 +233,25 @@ constexpr int kSumsBufferLen = kNumSums + 2;
 //              kinetic energy among them: one more live accumulator would
 //              cost the kModeSums variants registers); the last CTA
 //              publishes its own sums.
-constexpr int kModeLean = 0, kModeSums = 1, kModeFull = 2;
+// and, of pairs only,
+//   kModeField  the lean path with a force or Brinkman field.
+constexpr int kModeLean = 0, kModeSums = 1, kModeFull = 2, kModeField = 3;
 inline int step_mode(const StepArgs& a) {
     const bool plain = !a.force && !a.gamma && !a.rho_out && !a.check_finite;
     if (plain && !a.partials) return kModeLean;
     if (plain && !a.avg_out && !a.ke) return kModeSums;
     return kModeFull;
+}
+// of a pair: both steps share the variant (the fields' branches alone take
+// fewer registers than the full variant: three CTAs per SM).  Here kModeSums is the lean path
+// with the mass and momentum sums of the second step (and of the first when
+// it has accumulators) and, when it has somewhere to go, the moment store of
+// the second.
+inline int pair_mode(const PairArgs& p) {
+    const bool field = p.a.force || p.a.gamma, sums = p.a.partials || p.b.partials;
+    if (p.b.check_finite || p.a.ke || p.b.ke || (p.b.rho_out && !sums)) return kModeFull;
+    if (field) return sums ? kModeFull : kModeField;
+    return sums ? kModeSums : kModeLean;
 }
 // publishes the mass and momentum sums in acc (one accumulator set) into
 // sums / series
@@ -234,6 +278,47 @@ constexpr int kStageH16 = LBMX_TH16;
 // (a tile of more than 512 nodes gives each consumer thread several units)
 __host__ __device__ constexpr int step_tile_w(int elem_bytes) { return elem_bytes == 2 ? kStageW16 : kStageW; }
 __host__ __device__ constexpr int step_tile_h(int elem_bytes) { return elem_bytes == 2 ? kStageH16 : kStageH; }
+// Two-step kernel: tile shapes 0..3, CTAs resident per SM, ring depth.  A tile
+// computes the ring of nodes around it as well, so the largest tiles cost
+// least (64 x 12: 1.24 nodes of the first step per node, 32 x 8: 1.41 with
+// units of two) -- as long as three CTAs of two stages each fit an SM's
+// shared memory, since the collision's chain of dependent arithmetic wants
+// warps: an 8192^2 FP32 cavity takes 402 us a step with 64 x 12 and three
+// CTAs, 427 with 64 x 16 and two, 460 with 64 x 12 and two, 492 with 64 x 8
+// and four; FP16 391 with 64 x 20, 416 with 64 x 16 (single steps: 740 and
+// 414).  CM needs more than the 72 registers a thread has with three CTAs:
+// FP32 CM takes 64 x 16 and two (4096^2: 133.5 us, 134.9 with 64 x 12 and
+// three; 1024^2: 10.6 and 11.3).
+constexpr int kPairShapes = 4;
+__host__ __device__ constexpr int pair_w(int shape) { return shape < 2 ? 64 : 32; }
+__host__ __device__ constexpr int pair_h(int shape, int elem_bytes) {
+    return shape == 0 ? (elem_bytes == 4 ? 12 : 20) : shape == 3 ? 8 : 16;
+}
+__host__ __device__ constexpr int pair_ctas(int shape, int elem_bytes, int mode) {
+    return mode == kModeFull || (shape == 1 && elem_bytes == 4) ? 2 : 3;
+}
+constexpr int kPairStages = 2;
+// The shape of a lattice: large tiles when every resident CTA gets at least
+// two of them (16-bit's largest: three), 32 x 16 when every SM gets one, else
+// 32 x 8.  Measured per step, FP32: 256^2 vortex 2.6 us with 32 x 8, 2.7 with
+// 32 x 16; 384^2 cavity 3.5 and 3.1; 700^2 cavity 5.5 with 32 x 16, 5.9 with
+// 64 x 12; 1024^2 cavity 9.1 and 8.6; FP16 1024^2 8.9 with 64 x 16, 9.4 with
+// 64 x 20 and 10.1 with 32 x 16, 1536^2 17.7 and 16.7 with 64 x 20.
+inline int pair_shape(int nx, int ny, int elem_bytes, int op, int num_sms) {
+    const auto tiles = [&](int s) {
+        const int w = pair_w(s), h = pair_h(s, elem_bytes);
+        return (long long)((nx + w - 1) / w) * ((ny + h - 1) / h);
+    };
+    const auto slots = [&](int s) { return (long long)pair_ctas(s, elem_bytes, kModeLean) * num_sms; };
+    if (elem_bytes == 4) {
+        const int s = op == LBMX_CM ? 1 : 0;
+        if (tiles(s) >= 2 * slots(s)) return s;
+    } else {
+        if (tiles(0) >= 3 * slots(0)) return 0;
+        if (tiles(1) >= 2 * slots(1)) return 1;
+    }
+    return tiles(2) >= num_sms ? 2 : 3;
+}
 constexpr int kSpecialChunk = kConsumerWarps * 32;  // special nodes per work item (one per consumer thread)
 // guard elements before and after the population planes: staged row copies
 // reach one 16-byte chunk beyond a row segment on each side

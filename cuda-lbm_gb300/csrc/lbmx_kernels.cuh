@@ -218,12 +218,12 @@ __device__ __forceinline__ void node_force(const StepArgs& a, long long off, flo
 // (general_node).  Both step kernels, single-lattice and batched, make the
 // same choice for the same variant, so a lattice steps bit for bit alike
 // in either.
-template <typename T, int OP>
-__device__ __forceinline__ void general_node_body(const StepArgs& a, int x, int y, Acc v[kNumSums], uint32_t seed) {
-    const long long off = (long long)y * a.g.pitch + x;
-    float f[9];
-    unsigned outmask;
-    const uint8_t fl = gather_node<T>(a, x, y, f, &outmask);
+// node_collide is its part between the loads and the stores, shared with the
+// two-step kernel: f the node's post-stream, post-boundary populations on
+// entry and its post-collision populations on exit; its terms go into v when
+// `own`.
+template <int OP>
+__device__ __forceinline__ void node_collide(const StepArgs& a, long long off, float f[9], Acc v[kNumSums], bool own) {
     // macroscopics (macroscopics.cu:17-33): rho, j, raw Pi
     float rho = 0.f, jx = 0.f, jy = 0.f;
 #pragma unroll
@@ -251,13 +251,13 @@ __device__ __forceinline__ void general_node_body(const StepArgs& a, int x, int 
         a.u_out[off] = ux;
         a.u_out[a.g.plane + off] = uy;
     }
-    if (a.partials) {
+    if (own && a.partials) {
         // a node's terms in fixed point; the averages' terms only when
         // averages are produced
         v[0] += fix(rho);
         v[1] += fix(rho * ux);
         v[2] += fix(rho * uy);
-        if (a.ke) v[kSumKE] += fix(0.5f * rho * (ux * ux + uy * uy));
+        if (a.ke) v[kSumKE] += fix(0.5f * rho * fmaf(ux, ux, __fmul_rn(uy, uy)));  // rounded alike in every kernel
         if (a.avg_out) {
             v[4] += fix(rho * sqrtf(ux * ux + uy * uy));
             v[5] += fix(pimag);
@@ -274,6 +274,15 @@ __device__ __forceinline__ void general_node_body(const StepArgs& a, int x, int 
         const float jmag = sqrtf(ux * ux + uy * uy) * rho;
         collide_cm<float>(f, rho, rho, ux, uy, Fx, Fy, a.S, optimal_rate<float>(rho, jmag, pimag, a.avg), true);
     }
+}
+
+template <typename T, int OP>
+__device__ __forceinline__ void general_node_body(const StepArgs& a, int x, int y, Acc v[kNumSums], uint32_t seed) {
+    const long long off = (long long)y * a.g.pitch + x;
+    float f[9];
+    unsigned outmask;
+    const uint8_t fl = gather_node<T>(a, x, y, f, &outmask);
+    node_collide<OP>(a, off, f, v, true);
     store_post_collision<T>(a, x, y, f, outmask, fl, seed);
 }
 
@@ -395,32 +404,24 @@ __device__ __forceinline__ void stage_issue(const StepArgs& a, const CUtensorMap
 // accumulators an interior-path variant (step_mode) touches
 __host__ __device__ constexpr int mode_sums(int mode) { return mode == kModeLean ? 0 : (mode == kModeSums ? 3 : 6); }
 
-// Collide two staged interior nodes (x0, x0+1) of row y and store them in place.
-template <typename T, int OP, int P, int TW = kStageW, int TH = kStageH, int MODE = kModeFull>
-__device__ __forceinline__ void interior_unit(const StepArgs& a, const T* sbuf, int r, int lx, int x0, int y,
-                                              Acc v[kNumSums], uint32_t seed, const float* ibf = nullptr) {
-    using St = Staging<T, TW, TH>;
-    const Geometry& g = a.g;
-    T* F = static_cast<T*>(a.f);
-    const long long off = (long long)y * g.pitch + x0;
-    const long long plane = g.plane;
-    // 16-bit storage: f holds the stored offsets f - w throughout (the
-    // collision works in offset form); FP32: f itself
+// Moments, sums and collision of two x-neighbouring interior nodes whose
+// first has plane offset `off`, shared by the step kernels: f their
+// post-stream populations on entry (16-bit storage: offsets f - w), their
+// post-collision populations on exit; their terms go into v when `own`, or,
+// with TERMS in kModeSums, are returned in mom {rho, rho ux, rho uy, ux, uy}
+// instead.
+template <typename T, int OP, int MODE, bool TERMS = false>
+__device__ __forceinline__ void unit_collide(const StepArgs& a, long long off, V2 f[9], Acc v[kNumSums], bool own,
+                                             const float* ibf, V2* mom = nullptr) {
     constexpr bool OFS = kOffset<T>;
-    V2 f[9];
-#pragma unroll
-    for (int q = 0; q < 9; q++) {
-        const bool shifted = P && CX(q) != 0;
-        const T* s = sbuf + q * St::SLAB + r * St::TWP + 2 * lx + (shifted ? St::A - CX(q) : St::A);
-        f[q].v = shifted ? Store<T>::ld2r_u(s) : Store<T>::ld2r(s);
-    }
+    const long long plane = a.g.plane;
     V2 rho = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7])) + f[8];
     const V2 drho = rho;                     // offset form: rho - 1, exactly
     if (OFS) rho = rho + splat(1.0f, rho);  // the weights sum to 1
     const V2 jx = (f[1] - f[3]) + ((f[5] + f[8]) - (f[6] + f[7]));
     const V2 jy = (f[2] - f[4]) + ((f[5] + f[6]) - (f[7] + f[8]));
     V2 Fx = {make_float2(a.body_fx, a.body_fx)}, Fy = {make_float2(a.body_fy, a.body_fy)};
-    if (MODE == kModeFull && a.force) {
+    if ((MODE == kModeFull || MODE == kModeField) && a.force) {
         Fx.v = *reinterpret_cast<const float2*>(a.force + off);
         Fy.v = *reinterpret_cast<const float2*>(a.force + plane + off);
     }
@@ -433,7 +434,8 @@ __device__ __forceinline__ void interior_unit(const StepArgs& a, const T* sbuf, 
     const V2 inv = vdiv(splat(1.0f, rho), rho);
     V2 ux = fma(0.5f * Fx, inv, jx * inv);
     V2 uy = fma(0.5f * Fy, inv, jy * inv);
-    if (MODE == kModeFull && a.gamma) brinkman<V2>(V2{*reinterpret_cast<const float2*>(a.gamma + off)}, rho, ux, uy, Fx, Fy);
+    if ((MODE == kModeFull || MODE == kModeField) && a.gamma)
+        brinkman<V2>(V2{*reinterpret_cast<const float2*>(a.gamma + off)}, rho, ux, uy, Fx, Fy);
     V2 pimag = splat(0.f, rho);
     if (OP == LBMX_CM_OPT || (MODE == kModeFull && a.partials && a.avg_out)) {
         // offset form: sum c_x^2 w = sum c_y^2 w = 1/3
@@ -447,7 +449,13 @@ __device__ __forceinline__ void interior_unit(const StepArgs& a, const T* sbuf, 
         *reinterpret_cast<float2*>(a.u_out + off) = ux.v;
         *reinterpret_cast<float2*>(a.u_out + plane + off) = uy.v;
     }
-    if (MODE == kModeSums || (MODE == kModeFull && a.partials)) {
+    if (TERMS && MODE == kModeSums) {
+        mom[0] = rho;
+        mom[1] = rho * ux;
+        mom[2] = rho * uy;
+        mom[3] = ux;
+        mom[4] = uy;
+    } else if (own && (MODE == kModeSums || (MODE == kModeFull && a.partials))) {
         // the unit's terms in fixed point, the two nodes' summed in FP32
         // first (a fixed pairing, so the sums stay the same bit for bit):
         // half the 64-bit conversions, which run on the narrow FP64 pipe;
@@ -477,6 +485,27 @@ __device__ __forceinline__ void interior_unit(const StepArgs& a, const T* sbuf, 
         const V2 jmag = rho * vsqrt(fma(ux, ux, uy * uy));
         collide_cm<V2, OFS>(f, rho, drho, ux, uy, Fx, Fy, a.S, optimal_rate<V2>(rho, jmag, pimag, a.avg), true);
     }
+}
+
+// Collide two staged interior nodes (x0, x0+1) of row y and store them in place.
+template <typename T, int OP, int P, int TW = kStageW, int TH = kStageH, int MODE = kModeFull>
+__device__ __forceinline__ void interior_unit(const StepArgs& a, const T* sbuf, int r, int lx, int x0, int y,
+                                              Acc v[kNumSums], uint32_t seed, const float* ibf = nullptr) {
+    using St = Staging<T, TW, TH>;
+    const Geometry& g = a.g;
+    T* F = static_cast<T*>(a.f);
+    const long long off = (long long)y * g.pitch + x0;
+    // 16-bit storage: f holds the stored offsets f - w throughout (the
+    // collision works in offset form); FP32: f itself
+    constexpr bool OFS = kOffset<T>;
+    V2 f[9];
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+        const bool shifted = P && CX(q) != 0;
+        const T* s = sbuf + q * St::SLAB + r * St::TWP + 2 * lx + (shifted ? St::A - CX(q) : St::A);
+        f[q].v = shifted ? Store<T>::ld2r_u(s) : Store<T>::ld2r(s);
+    }
+    unit_collide<T, OP, MODE>(a, off, f, v, true, ibf);
     // slot q of the downstream nodes x + c_q (parity 1) or the nodes' own
     // slot OPP(q) (parity 0): byte offsets of this launch, from the host
     char* base = reinterpret_cast<char*>(F + off);

@@ -1,0 +1,4 @@
+#include "lbmx_pair_kernels.cuh"
+namespace lbmx {
+LBMX_INSTANTIATE_PAIR(__half)
+}

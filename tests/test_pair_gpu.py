@@ -1,0 +1,134 @@
+"""Two steps in one launch against single steps, bit for bit: the pair runs
+the same per-node arithmetic and rounding, so populations, moments and sums
+agree exactly over every boundary, wrap, ragged size and storage it takes."""
+import numpy as np
+import pytest
+
+import cases as C
+
+pytestmark = pytest.mark.gpu
+
+# sizes around the 32 x 8 tiles of small lattices: smaller than one, a whole
+# number, one node more or less, several ragged ones
+SIZES = [(3, 3), (5, 40), (63, 15), (64, 16), (65, 17), (66, 18), (129, 33), (200, 47)]
+
+
+def porous(nx, ny, **kw):
+    """Scattered obstacles of every local boundary among fluid nodes (few
+    enough for pairs), a force field and a Brinkman field."""
+    c = C.taylor_green(nx, ny, nu=0.05, **kw)
+    r = np.random.default_rng(3)
+    c["flags"][:] = r.choice([C.FLUID, C.CYLINDER, C.HALFWAY_BB, C.MOVING_WALL_BB, C.BOUNCE_BACK], (ny, nx),
+                             p=[0.997, 0.0006, 0.0006, 0.0006, 0.0012])
+    c["wall_u"] = (0.03, 0.01)
+    c["force"] = 1e-5 * r.standard_normal((2, ny, nx))
+    c["gamma"] = r.uniform(0.0, 0.3, (ny, nx)).astype(np.float32)
+    return c
+
+
+def corners(nx, ny, **kw):
+    c = C.channel(nx, ny, inlet="parabolic", outlet="zouhe_p", **kw)
+    c["flags"][-1, 0], c["flags"][0, 0] = C.CORNER_TOP_LEFT, C.CORNER_BOTTOM_LEFT
+    return c
+
+
+def regularized(nx, ny, **kw):
+    c = C.cavity_regularized(nx, ny, **kw)
+    c["flags"][c["flags"] == C.REGULARIZED_BOUNCE_BACK_CORNER] = C.REGULARIZED_BOUNCE_BACK
+    return c
+
+
+def open_box(nx, ny, **kw):
+    """Fluid up to non-periodic edges: every edge node reads the edge store."""
+    return C.base(nx, ny, kw.pop("op"), 0.05, **kw)
+
+
+FLOWS = {"vortex": C.taylor_green, "cavity": C.cavity_moving_wall, "zouhe": C.cavity_zouhe, "poiseuille": C.poiseuille,
+         "corners": corners, "regularized": regularized, "porous": porous, "open": open_box}
+
+
+def lattices(c, storage, count=2):
+    out = [C.make_lattice(c, storage=storage) for _ in range(count)]
+    for L in out:
+        if "gamma" in c:
+            L.set_brinkman(c["gamma"])
+    return out
+
+
+def same(A, B):
+    assert A.t == B.t
+    np.testing.assert_array_equal(A.populations(), B.populations())
+    ra, ua, sa = A.moments()
+    rb, ub, sb = B.moments()
+    np.testing.assert_array_equal(ra, rb)
+    np.testing.assert_array_equal(ua, ub)
+    np.testing.assert_array_equal(sa, sb)
+
+
+@pytest.mark.parametrize("size", SIZES)
+@pytest.mark.parametrize("flow", sorted(FLOWS))
+def test_pairs_equal_single_steps(flow, size):
+    import lbmx
+    for k, (op, storage) in enumerate([(C.BGK, 0), (C.MRT, 1), (C.CM, 0), (C.CM, 2)]):
+        c = C.random_state(FLOWS[flow](size[0], size[1], op=op), seed=k)
+        A, B = lattices(c, storage)
+        # even and odd starts, odd counts, moments stored by a pair and by a single step
+        for n in (2, 5, 1, 4):
+            A.step(n)
+            for i in range(n):
+                B.step(1, flags=lbmx.STEP_STORE_MOMENTS if i == n - 1 else 0)
+            same(A, B)
+
+
+@pytest.mark.parametrize("flow", ["porous", "corners", "cavity"])
+@pytest.mark.parametrize("nx,ny,op,storage", [
+    (651, 130, C.MRT, 0),    # 32 x 16 tiles
+    (650, 129, C.BGK, 1),
+    (1301, 531, C.MRT, 0),   # 64 x 12
+    (1281, 496, C.CM, 0),    # 64 x 16
+    (1300, 701, C.BGK, 1),
+    (2001, 901, C.MRT, 1),   # 64 x 20
+])
+def test_larger_tiles(flow, nx, ny, op, storage):
+    import lbmx
+    A, B = lattices(C.random_state(FLOWS[flow](nx, ny, op=op), seed=9), storage)
+    for n in (4, 3):
+        A.step(n, flags=lbmx.STEP_STORE_MOMENTS | lbmx.STEP_SUMS)
+        for _ in range(n):
+            B.step(1)
+        same(A, B)
+
+
+@pytest.mark.parametrize("flags", [0, 1, 9, 3])
+def test_series_of_pairs(flags):
+    """Per-step sums through pinned memory (pairs) and pageable memory (single steps)."""
+    import torch
+    import lbmx
+    c = C.random_state(C.cavity_moving_wall(200, 47, op=C.MRT), seed=4)
+    A, B = lattices(c, 0)
+    width = 4 if flags & lbmx.STEP_KINETIC_ENERGY else 3
+    for n in (6, 3, 4):
+        got = torch.zeros((n, width), dtype=torch.float64).pin_memory()
+        A._check(A.lib.lbmx_step_sums(A.h, n, flags, got.data_ptr()))
+        want = B.step_sums(n, flags)
+        A.synchronize()
+        np.testing.assert_array_equal(got.numpy(), want)
+        np.testing.assert_array_equal(A.moments()[2], B.moments()[2])
+        A.step(1, flags=lbmx.STEP_SUMS)
+        B.step(1, flags=lbmx.STEP_SUMS)
+        np.testing.assert_array_equal(A.moments()[2], B.moments()[2])
+
+
+def test_flags_changed_between_pairs():
+    """A half-way wall turned bounce-back reads the edge-store values its
+    nodes had before, whichever buffers the pairs left the state in."""
+    c = C.random_state(C.cavity_moving_wall(70, 37, op=C.BGK), seed=5)
+    d = C.cavity_zouhe(70, 37, op=C.BGK)["flags"]
+    A, B = lattices(c, 0)
+    for fl in (c["flags"], d, c["flags"], d):
+        for L in (A, B):
+            L.set_flags(fl)
+        A.step(6)
+        for _ in range(6):
+            B.step(1)
+        same(A, B)
