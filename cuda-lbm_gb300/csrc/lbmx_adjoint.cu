@@ -38,7 +38,11 @@ namespace lbmx {
 namespace {
 
 // Threads per block of every adjoint kernel; the reverse kernel (about 100
-// registers) is bounded to five 128-thread blocks per SM.
+// registers) is bounded to five 128-thread blocks per SM.  Both kernels are
+// bound by instruction issue more than by memory (2048 x 1024 CM: reverse 107
+// us for 285 MB, a floor of 42 us at the measured copy rate; forward 37 us,
+// floor 22 to 31); with a 64-bit division for the coordinates, wrap tests on
+// every link and FP64 objective terms on every node they took 149 and 51 us.
 constexpr int kAdjBlock = 128;
 constexpr int kAdjReverseBlocksPerSm = 5;
 constexpr int kTan = 2;  // tangents per pass
@@ -69,6 +73,22 @@ __device__ __forceinline__ float adj_wall_term(const AdjArgs& a, int q, uint8_t 
     return 6.0f * WQ(q) * ((float)CX(q) * a.wall_ux + (float)CY(q) * a.wall_uy);
 }
 
+// Coordinates of a node by 32-bit division (n fits 31 bits; the 64-bit one
+// is a software routine), and whether none of its links leaves the domain or
+// wraps: such a node's neighbours are at one offset per direction for the
+// whole launch.
+struct AdjNode {
+    int x, y;
+    bool inner;
+};
+__device__ __forceinline__ AdjNode adj_node_at(const AdjGeom& g, uint32_t node) {
+    AdjNode d;
+    d.y = (int)(node / (uint32_t)g.nx);
+    d.x = (int)(node - (uint32_t)d.y * (uint32_t)g.nx);
+    d.inner = d.x > 0 && d.x < g.nx - 1 && d.y > 0 && d.y < g.ny - 1;
+    return d;
+}
+
 // node x + s * c_q (wrapped on periodic axes), or -1 outside the domain
 __device__ __forceinline__ long long adj_link(const AdjGeom& g, int x, int y, int q, int s) {
     int nx = x + s * CX(q), ny = y + s * CY(q);
@@ -83,13 +103,18 @@ __device__ __forceinline__ long long adj_link(const AdjGeom& g, int x, int y, in
     return (long long)ny * g.nx + nx;
 }
 
-// post-stream populations of node (x, y) from the previous post-collision state
-__device__ __forceinline__ void adj_gather(const AdjArgs& a, const float* pc, int x, int y, long long node, uint8_t fl,
-                                           float ps[9]) {
+// post-stream populations of a node from the previous post-collision state
+__device__ __forceinline__ void adj_gather(const AdjArgs& a, const float* pc, const AdjNode& d, uint32_t node,
+                                           uint8_t fl, float ps[9]) {
     const long long n = a.g.n;
+    if (d.inner) {
+#pragma unroll
+        for (int q = 0; q < 9; q++) ps[q] = (pc + (q * n - (CY(q) * a.g.nx + CX(q))))[node];
+        return;
+    }
 #pragma unroll
     for (int q = 0; q < 9; q++) {
-        const long long s = adj_link(a.g, x, y, q, -1);
+        const long long s = adj_link(a.g, d.x, d.y, q, -1);
         if (s >= 0) ps[q] = pc[q * n + s];
         else if (adj_halfway(fl)) ps[q] = pc[OPP(q) * n + node] - adj_wall_term(a, OPP(q), fl);
         else ps[q] = 0.0f;  // overwritten by the node's bounce-back (checked on the host)
@@ -504,7 +529,8 @@ __device__ __forceinline__ void adj_node_vjp(const AdjArgs& a, int x, int y, uin
         if (CY(q) == -1) jy -= f[q];
     }
     const float rho = drho + 1.0f;
-    const float ux0 = (jx + 0.5f * a.fx) / rho, uy0 = (jy + 0.5f * a.fy) / rho;
+    const float inv = 1.0f / rho;
+    const float ux0 = (jx + 0.5f * a.fx) * inv, uy0 = (jy + 0.5f * a.fy) * inv;
     const float sc = 1.0f / (0.5f * gm + 1.0f);
     const float ux = ux0 * sc, uy = uy0 * sc;
     const float Fx = a.fx - gm * rho * ux, Fy = a.fy - gm * rho * uy;
@@ -585,7 +611,7 @@ __device__ __forceinline__ void adj_node_vjp(const AdjArgs& a, int x, int y, uin
     const float b_ux0 = sc * b_ux, b_uy0 = sc * b_uy;
     b_gm += -0.5f * sc * sc * (ux0 * b_ux + uy0 * b_uy);
     // Guo correction: u0 = (j + F0 / 2) / rho
-    const float b_jx = b_ux0 / rho, b_jy = b_uy0 / rho;
+    const float b_jx = b_ux0 * inv, b_jy = b_uy0 * inv;
     b_fx += 0.5f * b_jx;
     b_fy += 0.5f * b_jy;
     b_rho += -(ux0 * b_jx + uy0 * b_jy);
@@ -628,14 +654,14 @@ __global__ void adj_init_kernel(AdjGeom g, const float* rho, const float* u, flo
 
 // grid averages of step t (CM_OPT), block sums
 __global__ void adj_avg_kernel(const AdjArgs a, const float* pc_prev, double* part) {
-    const long long node = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
     double v[3] = {0.0, 0.0, 0.0};
     if (node < a.g.n) {
-        const int y = (int)(node / a.g.nx), x = (int)(node - (long long)y * a.g.nx);
+        const AdjNode d = adj_node_at(a.g, node);
         const uint8_t fl = a.flags ? a.flags[node] : (uint8_t)0;
         float f[9];
-        adj_gather(a, pc_prev, x, y, node, fl, f);
-        adj_bc<float>(a.g, f, x, y, fl);
+        adj_gather(a, pc_prev, d, node, fl, f);
+        adj_bc<float>(a.g, f, d.x, d.y, fl);
         float t[3];
         adj_avg_terms<float>(f, a.gamma ? a.gamma[node] : 0.0f, a.fx, a.fy, t);
         v[0] = t[0];
@@ -649,23 +675,29 @@ __global__ void adj_avg_kernel(const AdjArgs a, const float* pc_prev, double* pa
 template <int OP>
 __global__ void adj_forward_kernel(const AdjArgs a, const float* pc_prev, float* pc_next, const float* avg,
                                    int objective, double* jnode, float* rho_out, float* u_out) {
-    const long long node = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
     if (node >= a.g.n) return;
     const long long n = a.g.n;
-    const int y = (int)(node / a.g.nx), x = (int)(node - (long long)y * a.g.nx);
+    const AdjNode d = adj_node_at(a.g, node);
     const uint8_t fl = a.flags ? a.flags[node] : (uint8_t)0;
     float f[9];
-    adj_gather(a, pc_prev, x, y, node, fl, f);
-    adj_bc<float>(a.g, f, x, y, fl);
+    adj_gather(a, pc_prev, d, node, fl, f);
+    adj_bc<float>(a.g, f, d.x, d.y, fl);
     float mom[3];
     const float av[3] = {avg ? avg[0] : 1.0f, avg ? avg[1] : 1.0f, avg ? avg[2] : 1.0f};
     adj_node<float, OP>(a, f, a.gamma ? a.gamma[node] : 0.0f, a.fx, a.fy, a.omega, a.S, av, mom);
 #pragma unroll
-    for (int q = 0; q < 9; q++) pc_next[q * n + node] = f[q];
+    for (int q = 0; q < 9; q++) (pc_next + q * n)[node] = f[q];
     if (objective && a.weights) {
-        const double term = (double)a.weights[node] * mom[0] + (double)a.weights[n + node] * (mom[0] * mom[1]) +
-                            (double)a.weights[2 * n + node] * (mom[0] * mom[2]);
-        jnode[node] += a.drag ? (double)(a.gamma ? a.gamma[node] : 0.0f) * term : term;
+        const float w0 = a.weights[node], w1 = (a.weights + n)[node], w2 = (a.weights + 2 * n)[node];
+        const float mx = mom[0] * mom[1], my = mom[0] * mom[2];
+        // a node without weight adds nothing (unless its moments are not
+        // finite): no FP64 arithmetic, on a pipe that was two thirds busy
+        // with it, and no read and write of its 8-byte sum
+        if (w0 != 0.0f || w1 != 0.0f || w2 != 0.0f || !isfinite(mom[0] + mx + my)) {
+            const double term = (double)w0 * mom[0] + (double)w1 * mx + (double)w2 * my;
+            jnode[node] += a.drag ? (double)(a.gamma ? a.gamma[node] : 0.0f) * term : term;
+        }
     }
     if (rho_out) {
         rho_out[node] = mom[0];
@@ -682,22 +714,27 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjReverseBlocksPerSm) adj_reverse
                                                                 const float* lam_next, float* lam_out,
                                                                 const float* avg, int objective, double* g_gamma,
                                                                 double* part, double* avg_part) {
-    const long long node = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
     float sums[3] = {0.f, 0.f, 0.f}, asums[3] = {0.f, 0.f, 0.f};
     if (node < a.g.n) {
         const long long n = a.g.n;
-        const int y = (int)(node / a.g.nx), x = (int)(node - (long long)y * a.g.nx);
+        const AdjNode d = adj_node_at(a.g, node);
         const uint8_t fl = a.flags ? a.flags[node] : (uint8_t)0;
         float mu[9];
+        if (lam_next && d.inner) {
 #pragma unroll
-        for (int q = 0; q < 9; q++) {
-            float m = 0.0f;
-            if (lam_next) {
-                const long long d = adj_link(a.g, x, y, q, 1);
-                if (d >= 0) m = lam_next[q * n + d];
-                else if (adj_halfway(fl)) m = lam_next[OPP(q) * n + node];
+            for (int q = 0; q < 9; q++) mu[q] = (lam_next + (q * n + CY(q) * a.g.nx + CX(q)))[node];
+        } else {
+#pragma unroll
+            for (int q = 0; q < 9; q++) {
+                float m = 0.0f;
+                if (lam_next) {
+                    const long long to = adj_link(a.g, d.x, d.y, q, 1);
+                    if (to >= 0) m = lam_next[q * n + to];
+                    else if (adj_halfway(fl)) m = lam_next[OPP(q) * n + node];
+                }
+                mu[q] = m;
             }
-            mu[q] = m;
         }
         // The collision conserves mass, so a Jacobian column sums to an
         // integer -- 0 for the parameters, 1 (or more where bounce-back copies
@@ -712,19 +749,18 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjReverseBlocksPerSm) adj_reverse
 #pragma unroll
         for (int q = 0; q < 9; q++) mu[q] -= c;
         float ps[9];
-        adj_gather(a, pc_prev, x, y, node, fl, ps);
+        adj_gather(a, pc_prev, d, node, fl, ps);
         float w[3] = {0.0f, 0.0f, 0.0f};
         if (objective && a.weights) {
-            w[0] = a.weights[node];
-            w[1] = a.weights[n + node];
-            w[2] = a.weights[2 * n + node];
+#pragma unroll
+            for (int k = 0; k < 3; k++) w[k] = (a.weights + k * n)[node];
         }
         const float gm = a.gamma ? a.gamma[node] : 0.0f;
         const float av[3] = {avg ? avg[0] : 1.0f, avg ? avg[1] : 1.0f, avg ? avg[2] : 1.0f};
         float lam[9], d_gamma;
-        adj_node_vjp<OP>(a, x, y, fl, ps, gm, mu, c, w, av, lam, &d_gamma, &sums[0], &sums[1], &sums[2], asums);
+        adj_node_vjp<OP>(a, d.x, d.y, fl, ps, gm, mu, c, w, av, lam, &d_gamma, &sums[0], &sums[1], &sums[2], asums);
 #pragma unroll
-        for (int q = 0; q < 9; q++) lam_out[q * n + node] = lam[q];
+        for (int q = 0; q < 9; q++) (lam_out + q * n)[node] = lam[q];
         g_gamma[node] += d_gamma;
     }
     adj_block_sum<3, float>(sums, part, true);
@@ -736,13 +772,13 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjReverseBlocksPerSm) adj_reverse
 
 // CM_OPT: lambda_t += (1/N) G . d(terms)/dps with G the reduced sensitivity
 __global__ void adj_avg_back_kernel(const AdjArgs a, const float* pc_prev, const double* G, float* lam_out) {
-    const long long node = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
     if (node >= a.g.n) return;
     const long long n = a.g.n;
-    const int y = (int)(node / a.g.nx), x = (int)(node - (long long)y * a.g.nx);
+    const AdjNode nd = adj_node_at(a.g, node);
     const uint8_t fl = a.flags ? a.flags[node] : (uint8_t)0;
     float ps[9];
-    adj_gather(a, pc_prev, x, y, node, fl, ps);
+    adj_gather(a, pc_prev, nd, node, fl, ps);
     const float inv_n = (float)(1.0 / (double)n);
     const float g0 = (float)G[0] * inv_n, g1 = (float)G[1] * inv_n, g2 = (float)G[2] * inv_n;
     const float gm = a.gamma ? a.gamma[node] : 0.0f;
@@ -756,31 +792,46 @@ __global__ void adj_avg_back_kernel(const AdjArgs a, const float* pc_prev, const
 #pragma unroll
             for (int k = 0; k < kTan; k++) f[q].d[k] = (p0 + k == q) ? 1.0f : 0.0f;
         }
-        adj_bc<R>(a.g, f, x, y, fl);
+        adj_bc<R>(a.g, f, nd.x, nd.y, fl);
         adj_avg_terms<R>(f, dconst<kTan>(gm), dconst<kTan>(a.fx), dconst<kTan>(a.fy), t);
 #pragma unroll
         for (int k = 0; k < kTan; k++) {
             const int q = p0 + k;
             if (q >= 9) break;
-            lam_out[q * n + node] += g0 * t[0].d[k] + g1 * t[1].d[k] + g2 * t[2].d[k];
+            (lam_out + q * n)[node] += g0 * t[0].d[k] + g1 * t[1].d[k] + g2 * t[2].d[k];
         }
     }
 }
 
-// out[c] = sum over `count` rows of part[row][c] (one block, fixed order)
-__global__ void adj_sum_kernel(const double* part, long long count, int C, double* out, int add) {
-    __shared__ double sh[kAdjBlock];
+// out[c] = sum over `count` rows of part[row][c], in two stages of fixed
+// order: block b of the first sums the rows r = b * kSumThreads + t (mod the
+// grid's threads), the last stage is one block.  (One block alone took
+// 2.18 ms over the 2 M node sums of a 2048 x 1024 objective, 40 us over the
+// 16 K block sums of a step's averages.)
+constexpr int kSumThreads = 256, kSumBlocks = 296;
+template <int C>
+__global__ void __launch_bounds__(kSumThreads) adj_sum_kernel(const double* part, long long count, double* out) {
+    __shared__ double sh[kSumThreads / 32][C];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double t[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) t[c] = 0.0;
+    const long long step = (long long)gridDim.x * kSumThreads;
+#pragma unroll 4
+    for (long long r = (long long)blockIdx.x * kSumThreads + threadIdx.x; r < count; r += step)
+#pragma unroll
+        for (int c = 0; c < C; c++) t[c] += part[r * C + c];
+#pragma unroll
     for (int c = 0; c < C; c++) {
-        double t = 0.0;
-        for (long long r = threadIdx.x; r < count; r += kAdjBlock) t += part[r * C + c];
-        sh[threadIdx.x] = t;
-        __syncthreads();
-        for (int s = kAdjBlock / 2; s > 0; s >>= 1) {
-            if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[c] = add ? out[c] + sh[0] : sh[0];
-        __syncthreads();
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t[c] += __shfl_down_sync(0xffffffffu, t[c], o);
+        if (lane == 0) sh[warp][c] = t[c];
+    }
+    __syncthreads();
+    if (threadIdx.x < C) {
+        double s = 0.0;
+        for (int w = 0; w < kSumThreads / 32; w++) s += sh[w][threadIdx.x];
+        out[(long long)blockIdx.x * C + threadIdx.x] = s;
     }
 }
 
@@ -815,9 +866,10 @@ struct lbmx_adjoint {
     float* weights = nullptr;
     float* pc0 = nullptr;   // initial post-collision state [9][n]
     float* ping[2] = {nullptr, nullptr};
-    float* ckpt = nullptr;  // [ncheck][9][n]
+    float* ckpt = nullptr;  // [ncheck - 1][9][n] (the first checkpoint is pc0)
     int ncheck_cap = 0;
-    float* seg = nullptr;   // [every + 1][9][n]
+    float* seg = nullptr;   // [every - 1][9][n] states after a segment's checkpoint
+    bool kept = false;      // seg holds the last segment of the last forward run
     float* lam[2] = {nullptr, nullptr};
     float* avg_hist = nullptr;  // [T + 1][3]
     int avg_cap = 0;
@@ -826,6 +878,7 @@ struct lbmx_adjoint {
     double* part = nullptr;     // [blocks][3]
     double* avg_part = nullptr; // [blocks][3]
     double* red = nullptr;      // [8] reductions
+    double* sum_part = nullptr; // [kSumBlocks][3] first-stage sums, after red
     float* rho_out = nullptr;
     float* u_out = nullptr;
     long long blocks = 0;
@@ -908,12 +961,21 @@ static cudaError_t op_dispatch(int op, Fn fn) {
 
 static unsigned grid_of(long long n) { return (unsigned)((n + kAdjBlock - 1) / kAdjBlock); }
 
+// sum of `count` rows of part[row][C] into out[C] (a->sum_part: the blocks' sums)
+template <int C>
+static cudaError_t launch_sum(lbmx_adjoint* a, const double* part, long long count, double* out) {
+    const unsigned blocks = (unsigned)std::min<long long>(kSumBlocks, (count + kSumThreads - 1) / kSumThreads);
+    double* first = blocks > 1 ? a->sum_part : out;
+    adj_sum_kernel<C><<<blocks, kSumThreads, 0, a->stream>>>(part, count, first);
+    if (blocks > 1) adj_sum_kernel<C><<<1, kSumThreads, 0, a->stream>>>(first, blocks, out);
+    return cudaGetLastError();
+}
+
 // averages of step t (CM_OPT) into avg_hist[t]
 static lbmx_status step_averages(lbmx_adjoint* a, const float* pc_prev, int t) {
     adj_avg_kernel<<<grid_of(a->n), kAdjBlock, 0, a->stream>>>(a->args, pc_prev, a->avg_part);
     ADJ_CUDA(a, cudaGetLastError());
-    adj_sum_kernel<<<1, kAdjBlock, 0, a->stream>>>(a->avg_part, a->blocks, 3, a->red, 0);
-    ADJ_CUDA(a, cudaGetLastError());
+    ADJ_CUDA(a, launch_sum<3>(a, a->avg_part, a->blocks, a->red));
     adj_mean_kernel<<<1, 1, 0, a->stream>>>(a->red, a->avg_hist + (size_t)3 * t, 1.0 / (double)a->n);
     ADJ_CUDA(a, cudaGetLastError());
     return LBMX_OK;
@@ -1009,10 +1071,11 @@ lbmx_status lbmx_adjoint_create(const lbmx_params* p, const uint8_t* flags, int3
         cudaMalloc((void**)&a->jnode, (size_t)a->n * sizeof(double)) != cudaSuccess ||
         cudaMalloc((void**)&a->part, (size_t)a->blocks * 3 * sizeof(double)) != cudaSuccess ||
         cudaMalloc((void**)&a->avg_part, (size_t)a->blocks * 3 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void**)&a->red, 8 * sizeof(double)) != cudaSuccess ||
+        cudaMalloc((void**)&a->red, (8 + 3 * kSumBlocks) * sizeof(double)) != cudaSuccess ||
         cudaMalloc((void**)&a->rho_out, (size_t)a->n * sizeof(float)) != cudaSuccess ||
         cudaMalloc((void**)&a->u_out, (size_t)2 * a->n * sizeof(float)) != cudaSuccess)
         return bail("cudaMalloc failed");
+    a->sum_part = a->red + 8;
     if (p->stream) {
         a->stream = (cudaStream_t)p->stream;
     } else {
@@ -1098,11 +1161,12 @@ lbmx_status lbmx_adjoint_forward(lbmx_adjoint* a, int32_t nsteps, double* object
     if (nsteps < 1) return afail(a, LBMX_ERR_INVALID_ARGUMENT, "lbmx_adjoint_forward: nsteps < 1");
     cudaSetDevice(a->p.device);
     const size_t state = (size_t)9 * a->n;
-    const int ncheck = (nsteps + a->every - 1) / a->every;  // states at t = 0, every, 2 every, ...
+    // checkpoints: the states at t = 0 (pc0 itself), every, 2 every, ...
+    const int ncheck = (nsteps + a->every - 1) / a->every;
     if (ncheck > a->ncheck_cap) {
         cudaFree(a->ckpt);
         a->ckpt = nullptr;
-        ADJ_CUDA(a, cudaMalloc((void**)&a->ckpt, (size_t)ncheck * state * sizeof(float)));
+        if (ncheck > 1) ADJ_CUDA(a, cudaMalloc((void**)&a->ckpt, (size_t)(ncheck - 1) * state * sizeof(float)));
         a->ncheck_cap = ncheck;
     }
     if (nsteps + 1 > a->avg_cap) {
@@ -1111,19 +1175,33 @@ lbmx_status lbmx_adjoint_forward(lbmx_adjoint* a, int32_t nsteps, double* object
         ADJ_CUDA(a, cudaMalloc((void**)&a->avg_hist, (size_t)3 * (nsteps + 1) * sizeof(float)));
         a->avg_cap = nsteps + 1;
     }
+    // The last segment's states stay in the segment buffer the backward run
+    // would recompute them into, where that buffer is there or the device
+    // has room for it to spare (a run that never goes backward needs none).
+    const size_t seg_bytes = (size_t)(a->every - 1) * state * sizeof(float);
+    if (!a->seg && seg_bytes) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < seg_bytes + total_b / 2 ||
+            cudaMalloc((void**)&a->seg, seg_bytes) != cudaSuccess)
+            cudaGetLastError();
+    }
+    const int last0 = (ncheck - 1) * a->every;
+    a->kept = a->seg != nullptr;
     ADJ_CUDA(a, cudaMemsetAsync(a->jnode, 0, (size_t)a->n * sizeof(double), a->stream));
-    ADJ_CUDA(a, cudaMemcpyAsync(a->ping[0], a->pc0, state * sizeof(float), cudaMemcpyDeviceToDevice, a->stream));
+    // each step writes its state where it is needed next: a checkpoint, the
+    // segment buffer or one of two scratch states
+    const float* prev = a->pc0;
     int cur = 0;
     for (int t = 1; t <= nsteps; t++) {
-        if ((t - 1) % a->every == 0)
-            ADJ_CUDA(a, cudaMemcpyAsync(a->ckpt + (size_t)((t - 1) / a->every) * state, a->ping[cur],
-                                        state * sizeof(float), cudaMemcpyDeviceToDevice, a->stream));
-        lbmx_status st = forward_step(a, a->ping[cur], a->ping[cur ^ 1], t, t >= a->first, t == nsteps);
+        float* next;
+        if (t < nsteps && t % a->every == 0) next = a->ckpt + (size_t)(t / a->every - 1) * state;
+        else if (t < nsteps && t > last0 && a->kept) next = a->seg + (size_t)(t - last0 - 1) * state;
+        else next = a->ping[cur ^= 1];
+        lbmx_status st = forward_step(a, prev, next, t, t >= a->first, t == nsteps);
         if (st != LBMX_OK) return st;
-        cur ^= 1;
+        prev = next;
     }
-    adj_sum_kernel<<<1, kAdjBlock, 0, a->stream>>>(a->jnode, a->n, 1, a->red, 0);
-    ADJ_CUDA(a, cudaGetLastError());
+    ADJ_CUDA(a, launch_sum<1>(a, a->jnode, a->n, a->red));
     double J = 0.0;
     ADJ_CUDA(a, cudaMemcpyAsync(&J, a->red, sizeof(double), cudaMemcpyDeviceToHost, a->stream));
     ADJ_CUDA(a, cudaStreamSynchronize(a->stream));
@@ -1139,7 +1217,8 @@ lbmx_status lbmx_adjoint_backward(lbmx_adjoint* a, float* grad_gamma, double* gr
         return afail(a, LBMX_ERR_NOT_INITIALIZED, "lbmx_adjoint_backward: run lbmx_adjoint_forward with these inputs first");
     cudaSetDevice(a->p.device);
     const size_t state = (size_t)9 * a->n;
-    if (!a->seg) ADJ_CUDA(a, cudaMalloc((void**)&a->seg, (size_t)(a->every + 1) * state * sizeof(float)));
+    if (!a->seg && a->every > 1)
+        ADJ_CUDA(a, cudaMalloc((void**)&a->seg, (size_t)(a->every - 1) * state * sizeof(float)));
     if (!a->lam[0]) {
         ADJ_CUDA(a, cudaMalloc((void**)&a->lam[0], state * sizeof(float)));
         ADJ_CUDA(a, cudaMalloc((void**)&a->lam[1], state * sizeof(float)));
@@ -1154,13 +1233,14 @@ lbmx_status lbmx_adjoint_backward(lbmx_adjoint* a, float* grad_gamma, double* gr
     bool first_rev = true;
     for (int c = ncheck - 1; c >= 0; c--) {
         const int t0 = c * a->every, t1 = std::min(T, t0 + a->every);
-        // recompute the segment's states pc_t0 .. pc_t1
-        ADJ_CUDA(a, cudaMemcpyAsync(a->seg, a->ckpt + (size_t)c * state, state * sizeof(float),
-                                    cudaMemcpyDeviceToDevice, a->stream));
-        for (int t = t0 + 1; t <= t1; t++) {
+        // the segment's states pc_t0 .. pc_{t1-1}: a checkpoint, then
+        // recomputed ones (the last segment's may be there from the forward run)
+        const float* base = c == 0 ? a->pc0 : a->ckpt + (size_t)(c - 1) * state;
+        const auto state_at = [&](int t) { return t == t0 ? base : a->seg + (size_t)(t - t0 - 1) * state; };
+        for (int t = t0 + 1; t < t1 && !(a->kept && c == ncheck - 1); t++) {
             const float* avg = opt ? a->avg_hist + (size_t)3 * t : nullptr;
-            const float* prev = a->seg + (size_t)(t - 1 - t0) * state;
-            float* next = a->seg + (size_t)(t - t0) * state;
+            const float* prev = state_at(t - 1);
+            float* next = a->seg + (size_t)(t - t0 - 1) * state;
             ADJ_CUDA(a, op_dispatch(a->p.op, [&](auto opc) {
                          adj_forward_kernel<decltype(opc)::value><<<grid_of(a->n), kAdjBlock, 0, a->stream>>>(
                              a->args, prev, next, avg, 0, nullptr, nullptr, nullptr);
@@ -1168,7 +1248,7 @@ lbmx_status lbmx_adjoint_backward(lbmx_adjoint* a, float* grad_gamma, double* gr
                      }));
         }
         for (int t = t1; t > t0; t--) {
-            const float* prev = a->seg + (size_t)(t - 1 - t0) * state;
+            const float* prev = state_at(t - 1);
             const float* avg = opt ? a->avg_hist + (size_t)3 * t : nullptr;
             const float* lam_next = first_rev ? nullptr : a->lam[li];
             float* lam_out = a->lam[li ^ 1];
@@ -1179,8 +1259,7 @@ lbmx_status lbmx_adjoint_backward(lbmx_adjoint* a, float* grad_gamma, double* gr
                          return cudaGetLastError();
                      }));
             if (opt) {
-                adj_sum_kernel<<<1, kAdjBlock, 0, a->stream>>>(a->avg_part, a->blocks, 3, a->red + 4, 0);
-                ADJ_CUDA(a, cudaGetLastError());
+                ADJ_CUDA(a, launch_sum<3>(a, a->avg_part, a->blocks, a->red + 4));
                 adj_avg_back_kernel<<<grid_of(a->n), kAdjBlock, 0, a->stream>>>(a->args, prev, a->red + 4, lam_out);
                 ADJ_CUDA(a, cudaGetLastError());
             }
@@ -1188,8 +1267,7 @@ lbmx_status lbmx_adjoint_backward(lbmx_adjoint* a, float* grad_gamma, double* gr
             first_rev = false;
         }
     }
-    adj_sum_kernel<<<1, kAdjBlock, 0, a->stream>>>(a->part, a->blocks, 3, a->red, 0);
-    ADJ_CUDA(a, cudaGetLastError());
+    ADJ_CUDA(a, launch_sum<3>(a, a->part, a->blocks, a->red));
     double g3[3];
     ADJ_CUDA(a, cudaMemcpyAsync(g3, a->red, sizeof(g3), cudaMemcpyDeviceToHost, a->stream));
     if (grad_gamma) {
