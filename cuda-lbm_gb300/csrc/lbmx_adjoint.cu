@@ -37,14 +37,16 @@
 namespace lbmx {
 namespace {
 
-// Threads per block of every adjoint kernel; the reverse kernel (about 100
-// registers) is bounded to five 128-thread blocks per SM.  Both kernels are
-// bound by instruction issue more than by memory (2048 x 1024 CM: reverse 107
-// us for 285 MB, a floor of 42 us at the measured copy rate; forward 37 us,
-// floor 22 to 31); with a 64-bit division for the coordinates, wrap tests on
-// every link and FP64 objective terms on every node they took 149 and 51 us.
+// Threads per block of every adjoint kernel, and resident blocks per SM the
+// reverse kernel's registers are bounded for.  Neither kernel reaches memory
+// speed: 2048 x 1024 CM, reverse 95 us for 285 MB (a floor of 42 us at the
+// measured copy rate; latency of its 20 loads a node with 16 warps an SM, two
+// nodes a thread in packed arithmetic: five blocks spill, three are 112 us;
+// one node a thread 107 us), forward 37 us (floor 22 to 31, instruction
+// issue).  With a 64-bit division for the coordinates, wrap tests on every
+// link and FP64 objective terms on every node they took 149 and 51 us.
 constexpr int kAdjBlock = 128;
-constexpr int kAdjReverseBlocksPerSm = 5;
+constexpr int kAdjReverseBlocks1 = 5, kAdjReverseBlocks2 = 4;  // one and two nodes a thread
 constexpr int kTan = 2;  // tangents per pass
 
 struct AdjGeom {
@@ -227,6 +229,51 @@ __device__ __forceinline__ void adj_block_sum(const V v[C], double* part, bool a
     }
 }
 
+// ---------------------------------------------------------------- two nodes
+// Two nodes' values in one register pair, for the reverse pass: arithmetic in
+// packed FP32x2 instructions, a product kept pending until the sum it goes
+// into, so that a * b + c is one FFMA2 as the compiler makes one FFMA of it
+// in the scalar code.
+struct W2 {
+    float2 v;
+};
+struct W2P {  // a * b, not yet rounded
+    float2 a, b;
+    __device__ __forceinline__ operator W2() const { return W2{__fmul2_rn(a, b)}; }
+};
+__device__ __forceinline__ float2 both(float s) { return make_float2(s, s); }
+__device__ __forceinline__ float2 neg2(float2 v) { return make_float2(-v.x, -v.y); }
+__device__ __forceinline__ W2P operator*(W2 a, W2 b) { return W2P{a.v, b.v}; }
+__device__ __forceinline__ W2P operator*(float a, W2 b) { return W2P{both(a), b.v}; }
+__device__ __forceinline__ W2P operator*(W2 a, float b) { return W2P{both(b), a.v}; }
+__device__ __forceinline__ W2P operator-(W2P p) { return W2P{neg2(p.a), p.b}; }
+__device__ __forceinline__ W2 operator-(W2 a) { return W2{neg2(a.v)}; }
+__device__ __forceinline__ W2 operator+(W2 a, W2 b) { return W2{__fadd2_rn(a.v, b.v)}; }
+__device__ __forceinline__ W2 operator+(W2 a, float b) { return W2{__fadd2_rn(a.v, both(b))}; }
+__device__ __forceinline__ W2 operator+(W2P a, W2 b) { return W2{__ffma2_rn(a.a, a.b, b.v)}; }
+__device__ __forceinline__ W2 operator+(W2 a, W2P b) { return b + a; }
+__device__ __forceinline__ W2 operator+(W2P a, W2P b) { return a + W2(b); }
+__device__ __forceinline__ W2 operator+(W2P a, float b) { return a + W2{both(b)}; }
+__device__ __forceinline__ W2 operator-(W2 a, W2 b) { return W2{__ffma2_rn(b.v, both(-1.0f), a.v)}; }
+__device__ __forceinline__ W2 operator-(W2 a, W2P b) { return -b + a; }
+__device__ __forceinline__ W2 operator-(W2P a, W2 b) { return a + -b; }
+__device__ __forceinline__ W2 operator-(W2P a, W2P b) { return -b + W2(a); }
+__device__ __forceinline__ W2 operator-(W2 a, float b) { return a + -b; }
+__device__ __forceinline__ W2 operator-(float a, W2 b) { return W2{both(a)} - b; }
+__device__ __forceinline__ W2& operator+=(W2& a, W2 b) { return a = a + b; }
+__device__ __forceinline__ W2& operator+=(W2& a, W2P b) { return a = a + b; }
+__device__ __forceinline__ W2& operator-=(W2& a, W2 b) { return a = a - b; }
+__device__ __forceinline__ W2& operator-=(W2& a, W2P b) { return a = a - b; }
+// lanes: the nodes of a value (one, or two)
+__device__ __forceinline__ float& lane_of(float& v, int) { return v; }
+__device__ __forceinline__ float& lane_of(W2& v, int h) { return h ? v.v.y : v.v.x; }
+__device__ __forceinline__ float lanes_sum(float v) { return v; }
+__device__ __forceinline__ float lanes_sum(W2 v) { return v.v.x + v.v.y; }
+__device__ __forceinline__ float recip(float v) { return 1.0f / v; }
+__device__ __forceinline__ W2 recip(W2 v) { return W2{make_float2(1.0f / v.v.x, 1.0f / v.v.y)}; }
+template <typename R>
+constexpr int kLanes = sizeof(R) / sizeof(float);
+
 // ---------------------------------------------------------------- reverse
 // The node's vector-Jacobian product in reverse mode, written out by hand
 // for BGK, MRT, CM and CM_OPT: one pass over the node's values, then their
@@ -242,57 +289,58 @@ __device__ __forceinline__ void adj_block_sum(const V v[C], double* part, bool a
 // (raw moments r from central moments c by the binomial shift by +u), the
 // collision's adjoints of rho, drho, u, F and S; b_f gets the raw-moment
 // part (the populations' own adjoints through m = M f)
-__device__ __forceinline__ void vjp_cm(const float f[9], float rho, float drho, float ux, float uy, float Fx, float Fy,
-                                       const float S[9], const float mu[9], float b_f[9], float& b_rho, float& b_drho,
-                                       float& b_ux, float& b_uy, float& b_Fx, float& b_Fy, float b_S[9]) {
+template <typename R>
+__device__ __forceinline__ void vjp_cm(const R f[9], R rho, R drho, R ux, R uy, R Fx, R Fy,
+                                       const float S[9], const R mu[9], R b_f[9], R& b_rho, R& b_drho,
+                                       R& b_ux, R& b_uy, R& b_Fx, R& b_Fy, R b_S[9]) {
     const float third = 1.0f / 3.0f;
     // forward: raw moments, central moments, relaxed central moments
-    const float m10 = (f[1] - f[3]) + ((f[5] + f[8]) - (f[6] + f[7]));
-    const float m01 = (f[2] - f[4]) + ((f[5] + f[6]) - (f[7] + f[8]));
-    const float m22 = (f[5] + f[6]) + (f[7] + f[8]);
-    const float m20 = (f[1] + f[3]) + m22;
-    const float m02 = (f[2] + f[4]) + m22;
-    const float m11 = (f[5] + f[7]) - (f[6] + f[8]);
-    const float m21 = (f[5] + f[6]) - (f[7] + f[8]);
-    const float m12 = (f[5] + f[8]) - (f[6] + f[7]);
-    const float ux2 = ux * ux, uy2 = uy * uy, uxy = ux * uy;
-    const float k10 = m10 - ux * rho;
-    const float k01 = m01 - uy * rho;
-    const float k20 = m20 - 2.0f * ux * m10 + ux2 * rho;
-    const float k02 = m02 - 2.0f * uy * m01 + uy2 * rho;
-    const float k11 = m11 - uy * m10 - ux * m01 + uxy * rho;
-    const float k21 = m21 - 2.0f * ux * m11 - uy * m20 + ux2 * m01 + 2.0f * uxy * m10 - ux2 * uy * rho - uy * third;
-    const float k12 = m12 - 2.0f * uy * m11 - ux * m02 + uy2 * m10 + 2.0f * uxy * m01 - ux * uy2 * rho - ux * third;
-    const float k22 = m22 - 2.0f * ux * m12 - 2.0f * uy * m21 + ux2 * m02 + uy2 * m20 + 4.0f * uxy * m11 -
+    const R m10 = (f[1] - f[3]) + ((f[5] + f[8]) - (f[6] + f[7]));
+    const R m01 = (f[2] - f[4]) + ((f[5] + f[6]) - (f[7] + f[8]));
+    const R m22 = (f[5] + f[6]) + (f[7] + f[8]);
+    const R m20 = (f[1] + f[3]) + m22;
+    const R m02 = (f[2] + f[4]) + m22;
+    const R m11 = (f[5] + f[7]) - (f[6] + f[8]);
+    const R m21 = (f[5] + f[6]) - (f[7] + f[8]);
+    const R m12 = (f[5] + f[8]) - (f[6] + f[7]);
+    const R ux2 = ux * ux, uy2 = uy * uy, uxy = ux * uy;
+    const R k10 = m10 - ux * rho;
+    const R k01 = m01 - uy * rho;
+    const R k20 = m20 - 2.0f * ux * m10 + ux2 * rho;
+    const R k02 = m02 - 2.0f * uy * m01 + uy2 * rho;
+    const R k11 = m11 - uy * m10 - ux * m01 + uxy * rho;
+    const R k21 = m21 - 2.0f * ux * m11 - uy * m20 + ux2 * m01 + 2.0f * uxy * m10 - ux2 * uy * rho - uy * third;
+    const R k12 = m12 - 2.0f * uy * m11 - ux * m02 + uy2 * m10 + 2.0f * uxy * m01 - ux * uy2 * rho - ux * third;
+    const R k22 = m22 - 2.0f * ux * m12 - 2.0f * uy * m21 + ux2 * m02 + uy2 * m20 + 4.0f * uxy * m11 -
                       2.0f * ux * uy2 * m10 - 2.0f * ux2 * uy * m01 + ux2 * uy2 * rho + (ux2 + uy2) * third;
-    const float ksum = k20 + k02, kdiff = k20 - k02;
-    const float c10 = (1.0f - S[1]) * k10 + (1.0f - 0.5f * S[1]) * Fx;
-    const float c01 = (1.0f - S[2]) * k01 + (1.0f - 0.5f * S[2]) * Fy;
-    const float t3 = ksum - S[3] * (ksum - (2.0f * third) * drho);
-    const float t4 = (1.0f - S[4]) * kdiff;
-    const float c11 = (1.0f - S[5]) * k11;
-    const float c21 = (1.0f - S[6]) * k21 + (1.0f - 0.5f * S[6]) * third * Fy;
-    const float c12 = (1.0f - S[7]) * k12 + (1.0f - 0.5f * S[7]) * third * Fx;
-    const float c20 = 0.5f * (t3 + t4), c02 = 0.5f * (t3 - t4), c00 = rho;
+    const R ksum = k20 + k02, kdiff = k20 - k02;
+    const R c10 = (1.0f - S[1]) * k10 + (1.0f - 0.5f * S[1]) * Fx;
+    const R c01 = (1.0f - S[2]) * k01 + (1.0f - 0.5f * S[2]) * Fy;
+    const R t3 = ksum - S[3] * (ksum - (2.0f * third) * drho);
+    const R t4 = (1.0f - S[4]) * kdiff;
+    const R c11 = (1.0f - S[5]) * k11;
+    const R c21 = (1.0f - S[6]) * k21 + (1.0f - 0.5f * S[6]) * third * Fy;
+    const R c12 = (1.0f - S[7]) * k12 + (1.0f - 0.5f * S[7]) * third * Fx;
+    const R c20 = 0.5f * (t3 + t4), c02 = 0.5f * (t3 - t4), c00 = rho;
     // reverse: populations <- raw moments (f0 = drho - r20 - r02 + r22, ...)
-    const float b_r22 = mu[0] - 0.5f * (mu[1] + mu[3] + mu[2] + mu[4]) + 0.25f * (mu[5] + mu[6] + mu[7] + mu[8]);
-    const float b_r20 = 0.5f * (mu[1] + mu[3]) - mu[0];
-    const float b_r02 = 0.5f * (mu[2] + mu[4]) - mu[0];
-    const float b_r10 = 0.5f * (mu[1] - mu[3]);
-    const float b_r01 = 0.5f * (mu[2] - mu[4]);
-    const float b_r12 = 0.5f * (mu[3] - mu[1]) + 0.25f * ((mu[5] + mu[8]) - (mu[6] + mu[7]));
-    const float b_r21 = 0.5f * (mu[4] - mu[2]) + 0.25f * ((mu[5] + mu[6]) - (mu[7] + mu[8]));
-    const float b_r11 = 0.25f * ((mu[5] + mu[7]) - (mu[6] + mu[8]));
+    const R b_r22 = mu[0] - 0.5f * (mu[1] + mu[3] + mu[2] + mu[4]) + 0.25f * (mu[5] + mu[6] + mu[7] + mu[8]);
+    const R b_r20 = 0.5f * (mu[1] + mu[3]) - mu[0];
+    const R b_r02 = 0.5f * (mu[2] + mu[4]) - mu[0];
+    const R b_r10 = 0.5f * (mu[1] - mu[3]);
+    const R b_r01 = 0.5f * (mu[2] - mu[4]);
+    const R b_r12 = 0.5f * (mu[3] - mu[1]) + 0.25f * ((mu[5] + mu[8]) - (mu[6] + mu[7]));
+    const R b_r21 = 0.5f * (mu[4] - mu[2]) + 0.25f * ((mu[5] + mu[6]) - (mu[7] + mu[8]));
+    const R b_r11 = 0.25f * ((mu[5] + mu[7]) - (mu[6] + mu[8]));
     b_drho += mu[0];
     // raw moments <- central moments (shift by +u)
-    const float b_c10 = b_r10 + 2.0f * ux * b_r20 + uy * b_r11 + 2.0f * uxy * b_r21 + uy2 * b_r12 + 2.0f * ux * uy2 * b_r22;
-    const float b_c01 = b_r01 + 2.0f * uy * b_r02 + ux * b_r11 + ux2 * b_r21 + 2.0f * uxy * b_r12 + 2.0f * ux2 * uy * b_r22;
-    const float b_c20 = b_r20 + uy * b_r21 + uy2 * b_r22;
-    const float b_c02 = b_r02 + ux * b_r12 + ux2 * b_r22;
-    const float b_c11 = b_r11 + 2.0f * ux * b_r21 + 2.0f * uy * b_r12 + 4.0f * uxy * b_r22;
-    const float b_c21 = b_r21 + 2.0f * uy * b_r22;
-    const float b_c12 = b_r12 + 2.0f * ux * b_r22;
-    const float b_c22 = b_r22;
+    const R b_c10 = b_r10 + 2.0f * ux * b_r20 + uy * b_r11 + 2.0f * uxy * b_r21 + uy2 * b_r12 + 2.0f * ux * uy2 * b_r22;
+    const R b_c01 = b_r01 + 2.0f * uy * b_r02 + ux * b_r11 + ux2 * b_r21 + 2.0f * uxy * b_r12 + 2.0f * ux2 * uy * b_r22;
+    const R b_c20 = b_r20 + uy * b_r21 + uy2 * b_r22;
+    const R b_c02 = b_r02 + ux * b_r12 + ux2 * b_r22;
+    const R b_c11 = b_r11 + 2.0f * ux * b_r21 + 2.0f * uy * b_r12 + 4.0f * uxy * b_r22;
+    const R b_c21 = b_r21 + 2.0f * uy * b_r22;
+    const R b_c12 = b_r12 + 2.0f * ux * b_r22;
+    const R b_c22 = b_r22;
     b_rho += ux * b_r10 + uy * b_r01 + ux2 * b_r20 + uy2 * b_r02 + uxy * b_r11 + ux2 * uy * b_r21 + ux * uy2 * b_r12 +
              ux2 * uy2 * b_r22;
     b_ux += c00 * b_r10 + (2.0f * c10 + 2.0f * ux * c00) * b_r20 + (c01 + uy * c00) * b_r11 +
@@ -306,39 +354,39 @@ __device__ __forceinline__ void vjp_cm(const float f[9], float rho, float drho, 
             (2.0f * c21 + 2.0f * uy * c20 + 4.0f * ux * c11 + 4.0f * uxy * c10 + 2.0f * ux2 * c01 +
              2.0f * ux2 * uy * c00 + 2.0f * uy * third) * b_r22;
     // central moments <- relaxation
-    const float b_t3 = 0.5f * (b_c20 + b_c02), b_t4 = 0.5f * (b_c20 - b_c02);
-    const float b_k10 = (1.0f - S[1]) * b_c10;
+    const R b_t3 = 0.5f * (b_c20 + b_c02), b_t4 = 0.5f * (b_c20 - b_c02);
+    const R b_k10 = (1.0f - S[1]) * b_c10;
     b_S[1] += -(k10 + 0.5f * Fx) * b_c10;
     b_Fx += (1.0f - 0.5f * S[1]) * b_c10;
-    const float b_k01 = (1.0f - S[2]) * b_c01;
+    const R b_k01 = (1.0f - S[2]) * b_c01;
     b_S[2] += -(k01 + 0.5f * Fy) * b_c01;
     b_Fy += (1.0f - 0.5f * S[2]) * b_c01;
-    const float b_ksum = (1.0f - S[3]) * b_t3;
+    const R b_ksum = (1.0f - S[3]) * b_t3;
     b_drho += (2.0f * third) * S[3] * b_t3;
     b_S[3] += -(ksum - (2.0f * third) * drho) * b_t3;
-    const float b_kdiff = (1.0f - S[4]) * b_t4;
+    const R b_kdiff = (1.0f - S[4]) * b_t4;
     b_S[4] += -kdiff * b_t4;
-    const float b_k20 = b_ksum + b_kdiff, b_k02 = b_ksum - b_kdiff;
-    const float b_k11 = (1.0f - S[5]) * b_c11;
+    const R b_k20 = b_ksum + b_kdiff, b_k02 = b_ksum - b_kdiff;
+    const R b_k11 = (1.0f - S[5]) * b_c11;
     b_S[5] += -k11 * b_c11;
-    const float b_k21 = (1.0f - S[6]) * b_c21;
+    const R b_k21 = (1.0f - S[6]) * b_c21;
     b_S[6] += -(k21 + (0.5f * third) * Fy) * b_c21;
     b_Fy += (1.0f - 0.5f * S[6]) * third * b_c21;
-    const float b_k12 = (1.0f - S[7]) * b_c12;
+    const R b_k12 = (1.0f - S[7]) * b_c12;
     b_S[7] += -(k12 + (0.5f * third) * Fx) * b_c12;
     b_Fx += (1.0f - 0.5f * S[7]) * third * b_c12;
-    const float b_k22 = (1.0f - S[8]) * b_c22;
+    const R b_k22 = (1.0f - S[8]) * b_c22;
     b_drho += (third * third) * S[8] * b_c22;
     b_S[8] += -(k22 - (third * third) * drho) * b_c22;
     // raw moments <- central moments (shift by -u)
-    const float b_m10 = b_k10 - 2.0f * ux * b_k20 - uy * b_k11 + 2.0f * uxy * b_k21 + uy2 * b_k12 - 2.0f * ux * uy2 * b_k22;
-    const float b_m01 = b_k01 - 2.0f * uy * b_k02 - ux * b_k11 + ux2 * b_k21 + 2.0f * uxy * b_k12 - 2.0f * ux2 * uy * b_k22;
-    const float b_m20 = b_k20 - uy * b_k21 + uy2 * b_k22;
-    const float b_m02 = b_k02 - ux * b_k12 + ux2 * b_k22;
-    const float b_m11 = b_k11 - 2.0f * ux * b_k21 - 2.0f * uy * b_k12 + 4.0f * uxy * b_k22;
-    const float b_m21 = b_k21 - 2.0f * uy * b_k22;
-    const float b_m12 = b_k12 - 2.0f * ux * b_k22;
-    const float b_m22 = b_k22 + b_m20 + b_m02;
+    const R b_m10 = b_k10 - 2.0f * ux * b_k20 - uy * b_k11 + 2.0f * uxy * b_k21 + uy2 * b_k12 - 2.0f * ux * uy2 * b_k22;
+    const R b_m01 = b_k01 - 2.0f * uy * b_k02 - ux * b_k11 + ux2 * b_k21 + 2.0f * uxy * b_k12 - 2.0f * ux2 * uy * b_k22;
+    const R b_m20 = b_k20 - uy * b_k21 + uy2 * b_k22;
+    const R b_m02 = b_k02 - ux * b_k12 + ux2 * b_k22;
+    const R b_m11 = b_k11 - 2.0f * ux * b_k21 - 2.0f * uy * b_k12 + 4.0f * uxy * b_k22;
+    const R b_m21 = b_k21 - 2.0f * uy * b_k22;
+    const R b_m12 = b_k12 - 2.0f * ux * b_k22;
+    const R b_m22 = b_k22 + b_m20 + b_m02;
     b_rho += -ux * b_k10 - uy * b_k01 + ux2 * b_k20 + uy2 * b_k02 + uxy * b_k11 - ux2 * uy * b_k21 -
              ux * uy2 * b_k12 + ux2 * uy2 * b_k22;
     b_ux += -rho * b_k10 + (2.0f * ux * rho - 2.0f * m10) * b_k20 + (uy * rho - m01) * b_k11 +
@@ -363,19 +411,20 @@ __device__ __forceinline__ void vjp_cm(const float f[9], float rho, float drho, 
 }
 
 // MRT (Lallemand-Luo basis, offset form, forced): as vjp_cm
-__device__ __forceinline__ void vjp_mrt(const float f[9], float rho, float drho, float ux, float uy, float Fx, float Fy,
-                                        const float S[9], bool quirk, const float mu[9], float b_f[9], float& b_rho,
-                                        float& b_drho, float& b_ux, float& b_uy, float& b_Fx, float& b_Fy,
-                                        float b_S[9]) {
+template <typename R>
+__device__ __forceinline__ void vjp_mrt(const R f[9], R rho, R drho, R ux, R uy, R Fx, R Fy,
+                                        const float S[9], bool quirk, const R mu[9], R b_f[9], R& b_rho,
+                                        R& b_drho, R& b_ux, R& b_uy, R& b_Fx, R& b_Fy,
+                                        R b_S[9]) {
     const float inv_norm[9] = {1.0f / 9.0f, 1.0f / 36.0f, 1.0f / 36.0f, 1.0f / 6.0f, 1.0f / 12.0f,
                                1.0f / 6.0f, 1.0f / 12.0f, 0.25f, 0.25f};
     // forward: moments, equilibrium moments, force moments
-    const float axis = (f[1] + f[2]) + (f[3] + f[4]);
-    const float diag = (f[5] + f[6]) + (f[7] + f[8]);
-    const float d13 = f[1] - f[3], d24 = f[2] - f[4];
-    const float d58 = f[5] + f[8], d67 = f[6] + f[7];
-    const float d56 = f[5] + f[6], d78 = f[7] + f[8];
-    float m[9], meq[9], Fm[9];
+    const R axis = (f[1] + f[2]) + (f[3] + f[4]);
+    const R diag = (f[5] + f[6]) + (f[7] + f[8]);
+    const R d13 = f[1] - f[3], d24 = f[2] - f[4];
+    const R d58 = f[5] + f[8], d67 = f[6] + f[7];
+    const R d56 = f[5] + f[6], d78 = f[7] + f[8];
+    R m[9], meq[9], Fm[9];
     m[1] = 2.0f * diag - 4.0f * f[0] - axis;
     m[2] = 4.0f * f[0] - 2.0f * axis + diag;
     m[3] = d13 + (d58 - d67);
@@ -384,8 +433,8 @@ __device__ __forceinline__ void vjp_mrt(const float f[9], float rho, float drho,
     m[6] = -2.0f * d24 + (d56 - d78);
     m[7] = (f[1] + f[3]) - (f[2] + f[4]);
     m[8] = (f[5] + f[7]) - (f[6] + f[8]);
-    const float uu = ux * ux + uy * uy;
-    const float rux = rho * ux, ruy = rho * uy;
+    const R uu = ux * ux + uy * uy;
+    const R rux = rho * ux, ruy = rho * uy;
     meq[1] = 3.0f * rho * uu - 2.0f * drho;
     meq[2] = drho - 3.0f * rho * uu;
     meq[3] = rux;
@@ -394,7 +443,7 @@ __device__ __forceinline__ void vjp_mrt(const float f[9], float rho, float drho,
     meq[6] = -ruy;
     meq[7] = rho * (ux * ux - uy * uy);
     meq[8] = rux * uy;
-    const float fu = Fx * ux + Fy * uy;
+    const R fu = Fx * ux + Fy * uy;
     Fm[1] = 6.0f * fu;
     Fm[2] = -6.0f * fu;
     Fm[3] = Fx;
@@ -404,11 +453,11 @@ __device__ __forceinline__ void vjp_mrt(const float f[9], float rho, float drho,
     Fm[7] = 2.0f * (Fx * ux - Fy * uy);
     Fm[8] = Fx * uy + Fy * ux;
     // reverse: populations <- scaled post-collision moments a
-    float b_a[9];
-    const float b_axis_out = (mu[1] + mu[3]) + (mu[2] + mu[4]);
-    const float b_diag_out = (mu[5] + mu[6]) + (mu[7] + mu[8]);
-    const float b_ax = mu[1] - mu[3], b_ay = mu[2] - mu[4];
-    const float b_px = (mu[5] + mu[8]) - (mu[6] + mu[7]), b_py = (mu[5] + mu[6]) - (mu[7] + mu[8]);
+    R b_a[9];
+    const R b_axis_out = (mu[1] + mu[3]) + (mu[2] + mu[4]);
+    const R b_diag_out = (mu[5] + mu[6]) + (mu[7] + mu[8]);
+    const R b_ax = mu[1] - mu[3], b_ay = mu[2] - mu[4];
+    const R b_px = (mu[5] + mu[8]) - (mu[6] + mu[7]), b_py = (mu[5] + mu[6]) - (mu[7] + mu[8]);
     b_a[0] = mu[0] + b_axis_out + b_diag_out;
     b_a[1] = -4.0f * mu[0] - b_axis_out + 2.0f * b_diag_out;
     b_a[2] = 4.0f * mu[0] - 2.0f * b_axis_out + b_diag_out;
@@ -420,17 +469,17 @@ __device__ __forceinline__ void vjp_mrt(const float f[9], float rho, float drho,
     b_a[8] = (mu[5] + mu[7]) - (mu[6] + mu[8]);
     b_drho += b_a[0] * (1.0f / 9.0f);
     // a_k = inv_k ((1 - S_k) m_k + S_k meq_k + (1 - S_k / 2) Fm_k)
-    float b_m[9], b_meq[9], b_Fm[9];
+    R b_m[9], b_meq[9], b_Fm[9];
 #pragma unroll
     for (int k = 1; k < 9; k++) {
-        const float b = inv_norm[k] * b_a[k];
+        const R b = inv_norm[k] * b_a[k];
         b_m[k] = (1.0f - S[k]) * b;
         b_meq[k] = S[k] * b;
         b_Fm[k] = (1.0f - 0.5f * S[k]) * b;
         b_S[k] += (meq[k] - m[k] - 0.5f * Fm[k]) * b;
     }
     // force moments
-    const float b_fu = 6.0f * (b_Fm[1] - b_Fm[2]);
+    const R b_fu = 6.0f * (b_Fm[1] - b_Fm[2]);
     b_Fx += ux * b_fu + b_Fm[3] + 2.0f * ux * b_Fm[7] + uy * b_Fm[8];
     b_Fy += uy * b_fu - b_Fm[6] - 2.0f * uy * b_Fm[7] + ux * b_Fm[8];
     if (quirk) {
@@ -443,19 +492,19 @@ __device__ __forceinline__ void vjp_mrt(const float f[9], float rho, float drho,
     b_ux += Fx * b_fu + 2.0f * Fx * b_Fm[7] + Fy * b_Fm[8];
     b_uy += Fy * b_fu - 2.0f * Fy * b_Fm[7] + Fx * b_Fm[8];
     // equilibrium moments
-    const float b_uu = 3.0f * rho * (b_meq[1] - b_meq[2]);
+    const R b_uu = 3.0f * rho * (b_meq[1] - b_meq[2]);
     b_rho += 3.0f * uu * (b_meq[1] - b_meq[2]) + (ux * ux - uy * uy) * b_meq[7];
     b_drho += b_meq[2] - 2.0f * b_meq[1];
-    const float b_rux = b_meq[3] - b_meq[4] + uy * b_meq[8];
-    const float b_ruy = b_meq[5] - b_meq[6];
+    const R b_rux = b_meq[3] - b_meq[4] + uy * b_meq[8];
+    const R b_ruy = b_meq[5] - b_meq[6];
     b_uy += rux * b_meq[8];
     b_ux += 2.0f * rho * ux * b_meq[7] + rho * b_rux + 2.0f * ux * b_uu;
     b_uy += -2.0f * rho * uy * b_meq[7] + rho * b_ruy + 2.0f * uy * b_uu;
     b_rho += ux * b_rux + uy * b_ruy;
     // populations <- moments
-    const float b_axis = -b_m[1] - 2.0f * b_m[2], b_diag = 2.0f * b_m[1] + b_m[2];
-    const float b_d13 = b_m[3] - 2.0f * b_m[4], b_d5867 = b_m[3] + b_m[4];
-    const float b_d24 = b_m[5] - 2.0f * b_m[6], b_d5678 = b_m[5] + b_m[6];
+    const R b_axis = -b_m[1] - 2.0f * b_m[2], b_diag = 2.0f * b_m[1] + b_m[2];
+    const R b_d13 = b_m[3] - 2.0f * b_m[4], b_d5867 = b_m[3] + b_m[4];
+    const R b_d24 = b_m[5] - 2.0f * b_m[6], b_d5678 = b_m[5] + b_m[6];
     b_f[0] += 4.0f * (b_m[2] - b_m[1]);
     b_f[1] += b_axis + b_d13 + b_m[7];
     b_f[3] += b_axis - b_d13 + b_m[7];
@@ -468,33 +517,34 @@ __device__ __forceinline__ void vjp_mrt(const float f[9], float rho, float drho,
 }
 
 // BGK (offset form, forced): as vjp_cm; b_om the omega adjoint
-__device__ __forceinline__ void vjp_bgk(const float f[9], float rho, float drho, float ux, float uy, float Fx, float Fy,
-                                        float omega, const float mu[9], float b_f[9], float& b_rho, float& b_drho,
-                                        float& b_ux, float& b_uy, float& b_Fx, float& b_Fy, float& b_om) {
-    const float uu = ux * ux + uy * uy;
+template <typename R>
+__device__ __forceinline__ void vjp_bgk(const R f[9], R rho, R drho, R ux, R uy, R Fx, R Fy,
+                                        float omega, const R mu[9], R b_f[9], R& b_rho, R& b_drho,
+                                        R& b_ux, R& b_uy, R& b_Fx, R& b_Fy, R& b_om) {
+    const R uu = ux * ux + uy * uy;
     const float pref = 1.0f - 0.5f * omega;
-    float b_uu = 0.0f, b_pref = 0.0f;
+    R b_uu{}, b_pref{};
 #pragma unroll
     for (int q = 0; q < 9; q++) {
         const float cx = (float)CX(q), cy = (float)CY(q);
-        const float cu = cx * ux + cy * uy;
-        const float brm1 = cu * (4.5f * cu + 3.0f) - 1.5f * uu;
-        const float feq = WQ(q) * (rho * brm1 + drho);
-        const float gx = 9.0f * cx * cu + 3.0f * (cx - ux);
-        const float gy = 9.0f * cy * cu + 3.0f * (cy - uy);
+        const R cu = cx * ux + cy * uy;
+        const R brm1 = cu * (4.5f * cu + 3.0f) - 1.5f * uu;
+        const R feq = WQ(q) * (rho * brm1 + drho);
+        const R gx = 9.0f * cx * cu + 3.0f * (cx - ux);
+        const R gy = 9.0f * cy * cu + 3.0f * (cy - uy);
         // fn = f + omega (feq - f) + w pref (gx Fx + gy Fy)
-        const float m = mu[q];
+        const R m = mu[q];
         b_f[q] += (1.0f - omega) * m;
         b_om += (feq - f[q]) * m;
         b_pref += WQ(q) * (gx * Fx + gy * Fy) * m;
-        const float b_gx = WQ(q) * pref * Fx * m, b_gy = WQ(q) * pref * Fy * m;
+        const R b_gx = WQ(q) * pref * Fx * m, b_gy = WQ(q) * pref * Fy * m;
         b_Fx += WQ(q) * pref * gx * m;
         b_Fy += WQ(q) * pref * gy * m;
-        const float b_feq = omega * m;
+        const R b_feq = omega * m;
         b_rho += WQ(q) * brm1 * b_feq;
         b_drho += WQ(q) * b_feq;
-        const float b_brm1 = WQ(q) * rho * b_feq;
-        const float b_cu = (9.0f * cu + 3.0f) * b_brm1 + 9.0f * (cx * b_gx + cy * b_gy);
+        const R b_brm1 = WQ(q) * rho * b_feq;
+        const R b_cu = (9.0f * cu + 3.0f) * b_brm1 + 9.0f * (cx * b_gx + cy * b_gy);
         b_uu += -1.5f * b_brm1;
         b_ux += cx * b_cu - 3.0f * b_gx;
         b_uy += cy * b_cu - 3.0f * b_gy;
@@ -504,22 +554,29 @@ __device__ __forceinline__ void vjp_bgk(const float f[9], float rho, float drho,
     b_uy += 2.0f * uy * b_uu;
 }
 
-// The whole node: bounce-back, macroscopics with the Guo and Brinkman
-// corrections, collision, objective.  lam[q] = d/dps_q; the parameter
-// derivatives are returned through d_gamma, d_omega, d_fx, d_fy, and for
-// CM_OPT the derivatives of the node's term by the three grid averages
-// through d_avg.
-template <int OP>
-__device__ __forceinline__ void adj_node_vjp(const AdjArgs& a, int x, int y, uint8_t fl, const float ps[9], float gm,
-                                             const float mu[9], float c, const float w[3], const float* avg,
-                                             float lam[9], float* d_gamma, float* d_omega, float* d_fx, float* d_fy,
-                                             float d_avg[3]) {
-    float f[9];
+// The whole node (R float) or two nodes (R W2): bounce-back, macroscopics with
+// the Guo and Brinkman corrections, collision, objective.  lam[q] =
+// d/dps_q; the parameter derivatives are returned through d_gamma, d_omega,
+// d_fx, d_fy, and for CM_OPT (one node) the derivatives of the node's term by
+// the three grid averages through d_avg.
+template <int OP, typename R>
+__device__ __forceinline__ void adj_node_vjp(const AdjArgs& a, const AdjNode* nd, const uint8_t* fl, const R ps[9], R gm,
+                                             const R mu[9], R c, const R w[3], const float* avg, R lam[9], R* d_gamma,
+                                             R* d_omega, R* d_fx, R* d_fy, float d_avg[3]) {
+    R f[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) f[q] = ps[q];
-    adj_bc<float>(a.g, f, x, y, fl);
+#pragma unroll
+    for (int h = 0; h < kLanes<R>; h++) {
+        if (fl[h] != LBMX_BOUNCE_BACK) continue;
+#pragma unroll
+        for (int i = 1; i < 9; i++) {  // adj_bc
+            const int xn = nd[h].x + CX(i), yn = nd[h].y + CY(i);
+            if (xn < 0 || xn >= a.g.nx || yn < 0 || yn >= a.g.ny) lane_of(f[OPP(i)], h) = lane_of(f[i], h);
+        }
+    }
     // macroscopics (adj_macro)
-    float drho = f[0], jx = 0.0f, jy = 0.0f;
+    R drho = f[0], jx{}, jy{};
 #pragma unroll
     for (int q = 1; q < 9; q++) {
         drho += f[q];
@@ -528,31 +585,34 @@ __device__ __forceinline__ void adj_node_vjp(const AdjArgs& a, int x, int y, uin
         if (CY(q) == 1) jy += f[q];
         if (CY(q) == -1) jy -= f[q];
     }
-    const float rho = drho + 1.0f;
-    const float inv = 1.0f / rho;
-    const float ux0 = (jx + 0.5f * a.fx) * inv, uy0 = (jy + 0.5f * a.fy) * inv;
-    const float sc = 1.0f / (0.5f * gm + 1.0f);
-    const float ux = ux0 * sc, uy = uy0 * sc;
-    const float Fx = a.fx - gm * rho * ux, Fy = a.fy - gm * rho * uy;
+    const R rho = drho + 1.0f;
+    const R inv = recip(rho);
+    const R ux0 = (jx + 0.5f * a.fx) * inv, uy0 = (jy + 0.5f * a.fy) * inv;
+    const R sc = recip(R(0.5f * gm + 1.0f));
+    const R ux = ux0 * sc, uy = uy0 * sc;
+    const R gmr = gm * rho;
+    const R Fx = a.fx - R(gmr * ux), Fy = a.fy - R(gmr * uy);
     // adjoints
-    float b_f[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    float b_S[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    float b_rho = 0.f, b_drho = 0.f, b_ux = 0.f, b_uy = 0.f, b_Fx = 0.f, b_Fy = 0.f, b_om = 0.f, b_gm = 0.f;
+    R b_f[9] = {}, b_S[9] = {};
+    R b_rho{}, b_drho{}, b_ux{}, b_uy{}, b_Fx{}, b_Fy{}, b_om{}, b_gm{};
     // objective: w0 rho + w1 rho ux + w2 rho uy (drag: times gamma)
-    {
-        const float gscale = a.drag ? gm : 1.0f;
-        b_rho += gscale * (w[0] + w[1] * ux + w[2] * uy);
-        b_ux += gscale * w[1] * rho;
-        b_uy += gscale * w[2] * rho;
-        if (a.drag) b_gm += w[0] * rho + w[1] * rho * ux + w[2] * rho * uy;
+    if (a.drag) {
+        b_rho += gm * (w[0] + w[1] * ux + w[2] * uy);
+        b_ux += gm * w[1] * rho;
+        b_uy += gm * w[2] * rho;
+        b_gm += w[0] * rho + w[1] * rho * ux + w[2] * rho * uy;
+    } else {
+        b_rho += w[0] + w[1] * ux + w[2] * uy;
+        b_ux += w[1] * rho;
+        b_uy += w[2] * rho;
     }
-    if (OP == LBMX_BGK) {
-        vjp_bgk(f, rho, drho, ux, uy, Fx, Fy, a.omega, mu, b_f, b_rho, b_drho, b_ux, b_uy, b_Fx, b_Fy, b_om);
-    } else if (OP == LBMX_MRT) {
-        vjp_mrt(f, rho, drho, ux, uy, Fx, Fy, a.S, (a.quirks & LBMX_QUIRK_MRT_FORCE) != 0, mu, b_f, b_rho, b_drho,
-                b_ux, b_uy, b_Fx, b_Fy, b_S);
-    } else if (OP == LBMX_CM) {
-        vjp_cm(f, rho, drho, ux, uy, Fx, Fy, a.S, mu, b_f, b_rho, b_drho, b_ux, b_uy, b_Fx, b_Fy, b_S);
+    if constexpr (OP == LBMX_BGK) {
+        vjp_bgk<R>(f, rho, drho, ux, uy, Fx, Fy, a.omega, mu, b_f, b_rho, b_drho, b_ux, b_uy, b_Fx, b_Fy, b_om);
+    } else if constexpr (OP == LBMX_MRT) {
+        vjp_mrt<R>(f, rho, drho, ux, uy, Fx, Fy, a.S, (a.quirks & LBMX_QUIRK_MRT_FORCE) != 0, mu, b_f, b_rho, b_drho,
+                   b_ux, b_uy, b_Fx, b_Fy, b_S);
+    } else if constexpr (OP == LBMX_CM) {
+        vjp_cm<R>(f, rho, drho, ux, uy, Fx, Fy, a.S, mu, b_f, b_rho, b_drho, b_ux, b_uy, b_Fx, b_Fy, b_S);
     } else {
         // CM_OPT: the higher-order rate hor = 1 / (3 ts + 1/2), ts the
         // clamped regression in rho, |j| = rho |u| and |Pi| over the grid
@@ -571,7 +631,7 @@ __device__ __forceinline__ void adj_node_vjp(const AdjArgs& a, int x, int y, uin
         float Sh[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) Sh[k] = k >= 6 ? hor : a.S[k];
-        vjp_cm(f, rho, drho, ux, uy, Fx, Fy, Sh, mu, b_f, b_rho, b_drho, b_ux, b_uy, b_Fx, b_Fy, b_S);
+        vjp_cm<float>(f, rho, drho, ux, uy, Fx, Fy, Sh, mu, b_f, b_rho, b_drho, b_ux, b_uy, b_Fx, b_Fy, b_S);
         const float b_hor = b_S[6] + b_S[7] + b_S[8];
         b_S[6] = b_S[7] = b_S[8] = 0.0f;
         const float b_ts = free ? -3.0f * hor * hor * b_hor : 0.0f;
@@ -603,40 +663,55 @@ __device__ __forceinline__ void adj_node_vjp(const AdjArgs& a, int x, int y, uin
     for (int k = 0; k < 9; k++)
         if ((a.omega_mask >> k) & 1u) b_om += b_S[k];
     // Brinkman: F = F0 - gamma rho u, u = sc u0
-    float b_fx = b_Fx, b_fy = b_Fy;
-    b_gm += -rho * (ux * b_Fx + uy * b_Fy);
-    b_rho += -gm * (ux * b_Fx + uy * b_Fy);
-    b_ux += -gm * rho * b_Fx;
-    b_uy += -gm * rho * b_Fy;
-    const float b_ux0 = sc * b_ux, b_uy0 = sc * b_uy;
-    b_gm += -0.5f * sc * sc * (ux0 * b_ux + uy0 * b_uy);
+    R b_fx = b_Fx, b_fy = b_Fy;
+    const R uF = ux * b_Fx + uy * b_Fy;
+    b_gm -= rho * uF;
+    b_rho -= gm * uF;
+    b_ux -= gmr * b_Fx;
+    b_uy -= gmr * b_Fy;
+    const R b_ux0 = sc * b_ux, b_uy0 = sc * b_uy;
+    b_gm -= 0.5f * sc * R(ux0 * b_ux0 + uy0 * b_uy0);
     // Guo correction: u0 = (j + F0 / 2) / rho
-    const float b_jx = b_ux0 * inv, b_jy = b_uy0 * inv;
+    const R b_jx = b_ux0 * inv, b_jy = b_uy0 * inv;
     b_fx += 0.5f * b_jx;
     b_fy += 0.5f * b_jy;
-    b_rho += -(ux0 * b_jx + uy0 * b_jy);
+    b_rho -= ux0 * b_jx + uy0 * b_jy;
     b_drho += b_rho;
 #pragma unroll
-    for (int q = 0; q < 9; q++) b_f[q] += b_drho + (float)CX(q) * b_jx + (float)CY(q) * b_jy;
+    for (int q = 0; q < 9; q++) {
+        R t = b_drho;
+        if (CX(q) == 1) t = t + b_jx;
+        if (CX(q) == -1) t = t - b_jx;
+        if (CY(q) == 1) t = t + b_jy;
+        if (CY(q) == -1) t = t - b_jy;
+        b_f[q] += t;
+    }
     // bounce-back: f[OPP i] = f[i] for the links leaving the domain, undone
     // in reverse order; the mean c of the post-collision adjoints goes
     // through the conserved mass, whose derivative is the number of copies
     // of each post-stream population
-    float cnt[9] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
-    if (fl == LBMX_BOUNCE_BACK) {
+#pragma unroll
+    for (int h = 0; h < kLanes<R>; h++) {
+        const float ch = lane_of(c, h);
+        if (fl[h] != LBMX_BOUNCE_BACK) {
+#pragma unroll
+            for (int q = 0; q < 9; q++) lane_of(lam[q], h) = lane_of(b_f[q], h) + ch;
+            continue;
+        }
+        float cnt[9] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
 #pragma unroll
         for (int i = 8; i >= 1; i--) {
-            const int xn = x + CX(i), yn = y + CY(i);
+            const int xn = nd[h].x + CX(i), yn = nd[h].y + CY(i);
             if (xn < 0 || xn >= a.g.nx || yn < 0 || yn >= a.g.ny) {
-                b_f[i] += b_f[OPP(i)];
-                b_f[OPP(i)] = 0.0f;
+                lane_of(b_f[i], h) += lane_of(b_f[OPP(i)], h);
+                lane_of(b_f[OPP(i)], h) = 0.0f;
                 cnt[i] += cnt[OPP(i)];
                 cnt[OPP(i)] = 0.0f;
             }
         }
-    }
 #pragma unroll
-    for (int q = 0; q < 9; q++) lam[q] = fmaf(c, cnt[q], b_f[q]);
+        for (int q = 0; q < 9; q++) lane_of(lam[q], h) = fmaf(ch, cnt[q], lane_of(b_f[q], h));
+    }
     *d_gamma = b_gm;
     *d_omega = b_om;
     *d_fx = b_fx;
@@ -709,32 +784,56 @@ __global__ void adj_forward_kernel(const AdjArgs a, const float* pc_prev, float*
 // Reverse of step t.  lam_next = lambda_{t+1} (null at the last step);
 // writes lambda_t; g_gamma[node] += dJ/dgamma; part[block] += (domega, dFx,
 // dFy); CM_OPT: avg_part[block] = this step's sensitivity to the averages.
+// A thread takes the nodes t and t + kAdjBlock of its block's 2 kAdjBlock
+// (both streams coalesced, whatever nx) in packed arithmetic; CM_OPT, whose
+// rate is clamped node by node, one node.
 template <int OP>
-__global__ void __launch_bounds__(kAdjBlock, kAdjReverseBlocksPerSm) adj_reverse_kernel(const AdjArgs a, const float* pc_prev,
-                                                                const float* lam_next, float* lam_out,
-                                                                const float* avg, int objective, double* g_gamma,
-                                                                double* part, double* avg_part) {
-    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
+using AdjReal = std::conditional_t<OP == LBMX_CM_OPT, float, W2>;
+template <int OP>
+constexpr int kAdjNodes = kLanes<AdjReal<OP>>;
+template <int OP>
+__global__ void __launch_bounds__(kAdjBlock, kAdjNodes<OP> == 2 ? kAdjReverseBlocks2 : kAdjReverseBlocks1)
+    adj_reverse_kernel(const AdjArgs a, const float* pc_prev, const float* lam_next, float* lam_out, const float* avg,
+                       int objective, double* g_gamma, double* part, double* avg_part) {
+    using R = AdjReal<OP>;
+    constexpr int N = kAdjNodes<OP>;
+    const long long n = a.g.n;
     float sums[3] = {0.f, 0.f, 0.f}, asums[3] = {0.f, 0.f, 0.f};
-    if (node < a.g.n) {
-        const long long n = a.g.n;
-        const AdjNode d = adj_node_at(a.g, node);
-        const uint8_t fl = a.flags ? a.flags[node] : (uint8_t)0;
-        float mu[9];
-        if (lam_next && d.inner) {
+    const uint32_t node0 = blockIdx.x * (N * kAdjBlock) + threadIdx.x;
+    if (node0 < n) {
+        AdjNode nd[N];
+        uint8_t fl[N];
+        R mu[9] = {}, ps[9] = {}, w[3] = {}, gm{};
+        double gg[N];
 #pragma unroll
-            for (int q = 0; q < 9; q++) mu[q] = (lam_next + (q * n + CY(q) * a.g.nx + CX(q)))[node];
-        } else {
+        for (int h = 0; h < N; h++) {
+            const uint32_t node = node0 + h * kAdjBlock;
+            nd[h] = AdjNode{1, 1, true};
+            fl[h] = 0;
+            if (node >= n) continue;
+            nd[h] = adj_node_at(a.g, node);
+            fl[h] = a.flags ? a.flags[node] : (uint8_t)0;
+            if (lam_next && nd[h].inner) {
 #pragma unroll
-            for (int q = 0; q < 9; q++) {
-                float m = 0.0f;
-                if (lam_next) {
-                    const long long to = adj_link(a.g, d.x, d.y, q, 1);
-                    if (to >= 0) m = lam_next[q * n + to];
-                    else if (adj_halfway(fl)) m = lam_next[OPP(q) * n + node];
+                for (int q = 0; q < 9; q++)
+                    lane_of(mu[q], h) = (lam_next + (q * n + CY(q) * a.g.nx + CX(q)))[node];
+            } else if (lam_next) {
+#pragma unroll
+                for (int q = 0; q < 9; q++) {
+                    const long long to = adj_link(a.g, nd[h].x, nd[h].y, q, 1);
+                    if (to >= 0) lane_of(mu[q], h) = lam_next[q * n + to];
+                    else if (adj_halfway(fl[h])) lane_of(mu[q], h) = lam_next[OPP(q) * n + node];
                 }
-                mu[q] = m;
             }
+            float g[9];
+            adj_gather(a, pc_prev, nd[h], node, fl[h], g);
+#pragma unroll
+            for (int q = 0; q < 9; q++) lane_of(ps[q], h) = g[q];
+            if (objective && a.weights)
+#pragma unroll
+                for (int k = 0; k < 3; k++) lane_of(w[k], h) = (a.weights + k * n)[node];
+            if (a.gamma) lane_of(gm, h) = a.gamma[node];
+            if (OP != LBMX_CM) gg[h] = g_gamma[node];  // (early where registers allow)
         }
         // The collision conserves mass, so a Jacobian column sums to an
         // integer -- 0 for the parameters, 1 (or more where bounce-back copies
@@ -742,26 +841,26 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjReverseBlocksPerSm) adj_reverse
         // q.  Propagating mu - mean(mu) and adding mean(mu) times that
         // integer keeps FP32 from cancelling mean(mu) against the rounding
         // of the Jacobian.
-        float c = 0.0f;
+        R c = mu[0];
 #pragma unroll
-        for (int q = 0; q < 9; q++) c += mu[q];
-        c *= 1.0f / 9.0f;
+        for (int q = 1; q < 9; q++) c += mu[q];
+        c = c * (1.0f / 9.0f);
 #pragma unroll
         for (int q = 0; q < 9; q++) mu[q] -= c;
-        float ps[9];
-        adj_gather(a, pc_prev, d, node, fl, ps);
-        float w[3] = {0.0f, 0.0f, 0.0f};
-        if (objective && a.weights) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) w[k] = (a.weights + k * n)[node];
-        }
-        const float gm = a.gamma ? a.gamma[node] : 0.0f;
         const float av[3] = {avg ? avg[0] : 1.0f, avg ? avg[1] : 1.0f, avg ? avg[2] : 1.0f};
-        float lam[9], d_gamma;
-        adj_node_vjp<OP>(a, d.x, d.y, fl, ps, gm, mu, c, w, av, lam, &d_gamma, &sums[0], &sums[1], &sums[2], asums);
+        R lam[9], d_gamma, d_omega, d_fx, d_fy;
+        adj_node_vjp<OP, R>(a, nd, fl, ps, gm, mu, c, w, av, lam, &d_gamma, &d_omega, &d_fx, &d_fy, asums);
 #pragma unroll
-        for (int q = 0; q < 9; q++) (lam_out + q * n)[node] = lam[q];
-        g_gamma[node] += d_gamma;
+        for (int h = 0; h < N; h++) {
+            const uint32_t node = node0 + h * kAdjBlock;
+            if (node >= n) continue;
+#pragma unroll
+            for (int q = 0; q < 9; q++) (lam_out + q * n)[node] = lane_of(lam[q], h);
+            g_gamma[node] = (OP != LBMX_CM ? gg[h] : g_gamma[node]) + (double)lane_of(d_gamma, h);
+        }
+        sums[0] = lanes_sum(d_omega);
+        sums[1] = lanes_sum(d_fx);
+        sums[2] = lanes_sum(d_fy);
     }
     adj_block_sum<3, float>(sums, part, true);
     if (OP == LBMX_CM_OPT) {
@@ -960,6 +1059,12 @@ static cudaError_t op_dispatch(int op, Fn fn) {
 }
 
 static unsigned grid_of(long long n) { return (unsigned)((n + kAdjBlock - 1) / kAdjBlock); }
+
+// blocks of the reverse kernel (and rows of its partial sums)
+static unsigned reverse_blocks(const lbmx_adjoint* a) {
+    const int nodes = kAdjBlock * (a->p.op == LBMX_CM_OPT ? kAdjNodes<LBMX_CM_OPT> : kAdjNodes<LBMX_CM>);
+    return (unsigned)((a->n + nodes - 1) / nodes);
+}
 
 // sum of `count` rows of part[row][C] into out[C] (a->sum_part: the blocks' sums)
 template <int C>
@@ -1254,12 +1359,13 @@ lbmx_status lbmx_adjoint_backward(lbmx_adjoint* a, float* grad_gamma, double* gr
             float* lam_out = a->lam[li ^ 1];
             const int objective = t >= a->first ? 1 : 0;
             ADJ_CUDA(a, op_dispatch(a->p.op, [&](auto opc) {
-                         adj_reverse_kernel<decltype(opc)::value><<<grid_of(a->n), kAdjBlock, 0, a->stream>>>(
+                         adj_reverse_kernel<decltype(opc)::value>
+                             <<<reverse_blocks(a), kAdjBlock, 0, a->stream>>>(
                              a->args, prev, lam_next, lam_out, avg, objective, a->g_gamma, a->part, a->avg_part);
                          return cudaGetLastError();
                      }));
             if (opt) {
-                ADJ_CUDA(a, launch_sum<3>(a, a->avg_part, a->blocks, a->red + 4));
+                ADJ_CUDA(a, launch_sum<3>(a, a->avg_part, reverse_blocks(a), a->red + 4));
                 adj_avg_back_kernel<<<grid_of(a->n), kAdjBlock, 0, a->stream>>>(a->args, prev, a->red + 4, lam_out);
                 ADJ_CUDA(a, cudaGetLastError());
             }
@@ -1267,7 +1373,7 @@ lbmx_status lbmx_adjoint_backward(lbmx_adjoint* a, float* grad_gamma, double* gr
             first_rev = false;
         }
     }
-    ADJ_CUDA(a, launch_sum<3>(a, a->part, a->blocks, a->red));
+    ADJ_CUDA(a, launch_sum<3>(a, a->part, reverse_blocks(a), a->red));
     double g3[3];
     ADJ_CUDA(a, cudaMemcpyAsync(g3, a->red, sizeof(g3), cudaMemcpyDeviceToHost, a->stream));
     if (grad_gamma) {
