@@ -147,3 +147,23 @@ def test_tangent_rejects_what_it_does_not_differentiate():
     with pytest.raises(lbmx.LbmxError) as e:
         t.run(1)  # no state yet
     assert e.value.code == 5
+
+
+@pytest.mark.parametrize("op", [C.BGK, C.MRT, C.CM])
+def test_markers_off_walls_and_across_blocks(op):
+    """The step overlaps its IBM kernel except on the patch nodes: bodies at
+    the blocks' edges, beside the walls and in the last block give the same
+    drag and lift as the engine's own steps, with another tangent's smaller
+    body set in between."""
+    for centre, r, n in (((32.0, 16.0), 5.5, 24), ((95.7, 31.6), 6.0, 40), ((104.0, 37.5), 4.0, 12)):
+        c = cylinder(op)
+        c["markers"] = C.cylinder_markers(centre[0], centre[1], r, n)
+        t = tangent_of(c, lbmx.TANGENT_U_BC)
+        small = dict(c, markers=C.cylinder_markers(50.0, 20.0, 3.0, 6))
+        other = tangent_of(small, lbmx.TANGENT_U_BC)
+        got = t.run(60)
+        L = C.make_lattice(c)
+        want = L.step_forces(60)
+        scale = np.abs(want).max()
+        assert np.abs(got[:, :2] - want).max() <= 1e-4 * scale
+        assert np.isfinite(other.run(3)).all()
