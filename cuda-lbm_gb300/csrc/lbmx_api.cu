@@ -396,17 +396,60 @@ static lbmx_status rebuild_special(lbmx_handle* h, bool pair_lists = true) {
     return LBMX_OK;
 }
 
-// A staged tile whose copies never completed (bit 1 of the error word) is a
-// hard failure of the steps since the last check; the word is cleared.
-static lbmx_status check_pipeline(lbmx_handle* h) {
-    unsigned int w = 0;
-    LBMX_CUDA(h, cudaMemcpyAsync(&w, h->error_word, sizeof(w), cudaMemcpyDeviceToHost, h->stream));
-    LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (w & 2u) {
-        LBMX_CUDA(h, cudaMemsetAsync(h->error_word, 0, sizeof(w), h->stream));
-        return fail(h, LBMX_ERR_CUDA, "step kernel: a shared-memory staging wait gave up; results are invalid");
+// The stored moments into the caller's dense device fields (either may be
+// null), and the sums and the error word into the handle's pinned mailbox: a
+// readback is one launch and one wait (three row copies, two small copies
+// and three waits took 40 us of a 64^2 step-and-read call, and the row
+// copies 0.7 ms of 8192^2 fields: 805 MB, now at copy speed).  A warp takes
+// a row, four nodes a lane where rows start on 16 bytes in both.
+struct ReadbackArgs {
+    const float* src;  // rho, ux, uy planes
+    long long plane;
+    int nx, ny, pitch;
+    float* rho;
+    float* u;
+    const double* sums;
+    const unsigned int* error_word;
+    double* mail;      // [4] sums 0..2, then the error word
+};
+constexpr int kReadbackRows = 8;
+__global__ void __launch_bounds__(32 * kReadbackRows) readback_kernel(const ReadbackArgs a, int vec) {
+    if (blockIdx.x == 0 && threadIdx.x < 3 && threadIdx.y == 0) a.mail[threadIdx.x] = a.sums[threadIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x == 3 && threadIdx.y == 0) a.mail[3] = (double)*a.error_word;
+    const int row = (a.rho ? 0 : a.ny) + (int)(blockIdx.x * kReadbackRows + threadIdx.y);
+    if (row >= (a.u ? 3 * a.ny : a.ny)) return;
+    const int c = row / a.ny, y = row - c * a.ny;
+    const float* s = a.src + c * a.plane + (long long)y * a.pitch;
+    const long long n = (long long)a.nx * a.ny;
+    float* d = (c == 0 ? a.rho : a.u + (c - 1) * n) + (long long)y * a.nx;
+    if (vec) {
+        const float4* s4 = reinterpret_cast<const float4*>(s);
+        float4* d4 = reinterpret_cast<float4*>(d);
+#pragma unroll 4
+        for (int i = threadIdx.x; i < a.nx / 4; i += 32) d4[i] = s4[i];
+    } else {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < a.nx; i += 32) d[i] = s[i];
     }
-    return LBMX_OK;
+}
+
+// Device memory the handle's kernels may write (null: nothing to write).
+static bool device_writable(const lbmx_handle* h, const void* p) {
+    if (!p) return true;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == h->p.device);
+}
+
+// A staged tile whose copies never completed (bit 1 of the error word w) is a
+// hard failure of the steps since the last check; the word is cleared.
+static lbmx_status check_word(lbmx_handle* h, unsigned int w) {
+    if (!(w & 2u)) return LBMX_OK;
+    LBMX_CUDA(h, cudaMemsetAsync(h->error_word, 0, sizeof(w), h->stream));
+    return fail(h, LBMX_ERR_CUDA, "step kernel: a shared-memory staging wait gave up; results are invalid");
 }
 
 // parity and rest-population plane of step index s (1-based)
@@ -485,6 +528,7 @@ void lbmx_destroy(lbmx_handle* h) {
     cudaFree(h->force); cudaFree(h->gamma); cudaFree(h->rho_out); cudaFree(h->pop_out); cudaFree(h->raw_sums);
     cudaFree(h->special_units); cudaFree(h->bits_buf); cudaFree(h->special_units0); cudaFree(h->bits0_buf);
     cudaFree(h->tile_order);
+    cudaFreeHost(h->mail);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
     cudaSetDevice(cur);
     delete h;
@@ -579,6 +623,11 @@ lbmx_status lbmx_create(const lbmx_params* p, lbmx_handle** out) {
     // work counters, the averages, the last-block counter and the error word
     const size_t words = (size_t)(kAccSets * kAccPerSet + kSumsBufferLen + 4) * 8 + 5 * 4;
     ALLOC(h->words, words);
+    if (cudaMallocHost((void**)&h->mail, 4 * sizeof(double)) != cudaSuccess) {
+        fail(nullptr, LBMX_ERR_OUT_OF_MEMORY, "lbmx_create: cudaMallocHost failed");
+        lbmx_destroy(h);
+        return LBMX_ERR_OUT_OF_MEMORY;
+    }
     h->partials = static_cast<double*>(h->words);
     h->sums = h->partials + kAccSets * kAccPerSet;
     h->tile_counter = reinterpret_cast<unsigned long long*>(h->sums + kSumsBufferLen);
@@ -1124,24 +1173,35 @@ lbmx_status lbmx_moments(lbmx_handle* h, float* rho, float* u, double* sums3) {
     cudaSetDevice(h->p.device);
     const Geometry& g = h->g;
     const long long n = (long long)g.nx * g.ny;
-    if (rho)
+    // device fields by the readback kernel, host fields by row copies
+    ReadbackArgs a;
+    memset(&a, 0, sizeof(a));
+    a.src = h->rho_out;
+    a.plane = g.plane;
+    a.nx = g.nx;
+    a.ny = g.ny;
+    a.pitch = g.pitch;
+    a.sums = h->sums;
+    a.error_word = h->error_word;
+    a.mail = h->mail;
+    if (device_writable(h, rho)) a.rho = rho;
+    else
         LBMX_CUDA(h, cudaMemcpy2DAsync(rho, g.nx * sizeof(float), h->rho_out, g.pitch * sizeof(float),
                                        g.nx * sizeof(float), g.ny, cudaMemcpyDefault, h->stream));
-    if (u)
+    if (device_writable(h, u)) a.u = u;
+    else
         for (int c = 0; c < 2; c++)
             LBMX_CUDA(h, cudaMemcpy2DAsync(u + c * n, g.nx * sizeof(float), h->u_out + c * g.plane,
                                            g.pitch * sizeof(float), g.nx * sizeof(float), g.ny, cudaMemcpyDefault,
                                            h->stream));
-    if (sums3) {
-        double s[6];
-        LBMX_CUDA(h, cudaMemcpyAsync(s, h->sums, sizeof(s), cudaMemcpyDeviceToHost, h->stream));
-        LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
-        sums3[0] = s[0];
-        sums3[1] = s[1];
-        sums3[2] = s[2];
-    }
+    const int rows = (a.rho ? g.ny : 0) + (a.u ? 2 * g.ny : 0);
+    const int vec = g.nx % 4 == 0 && reinterpret_cast<uintptr_t>(a.rho) % 16 == 0 && reinterpret_cast<uintptr_t>(a.u) % 16 == 0;
+    readback_kernel<<<std::max(1, (rows + kReadbackRows - 1) / kReadbackRows), dim3(32, kReadbackRows), 0, h->stream>>>(a, vec);
+    LBMX_CUDA(h, cudaGetLastError());
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
-    return check_pipeline(h);
+    if (sums3)
+        for (int k = 0; k < 3; k++) sums3[k] = h->mail[k];
+    return check_word(h, (unsigned int)h->mail[3]);
 }
 
 lbmx_status lbmx_get_populations(lbmx_handle* h, float* out) {
@@ -1549,8 +1609,10 @@ lbmx_status lbmx_write_vti(lbmx_handle* h, const char* path) {
 lbmx_status lbmx_synchronize(lbmx_handle* h) {
     if (!h) return fail(h, LBMX_ERR_INVALID_ARGUMENT, "lbmx_synchronize: NULL handle");
     cudaSetDevice(h->p.device);
+    unsigned int* w = reinterpret_cast<unsigned int*>(h->mail);
+    LBMX_CUDA(h, cudaMemcpyAsync(w, h->error_word, sizeof(*w), cudaMemcpyDeviceToHost, h->stream));
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
-    return check_pipeline(h);
+    return check_word(h, *w);
 }
 
 const char* lbmx_last_error(lbmx_handle* h) { return h ? h->err : g_create_err; }

@@ -71,6 +71,7 @@ struct lbmx_handle {
     int nspecial = 0, special_chunks = 0, tiles_x = 0, tiles_y = 0, num_ctas = 0, num_sms = 1;
     void* f_alloc = nullptr;  // population allocation (f and f2) including the guard elements
     float* edge_alloc = nullptr;  // aux, edge and edge2
+    double* mail = nullptr;       // pinned host words a readback leaves sums and error word in
     void* words = nullptr;        // partials, sums, counters, averages, error word
     // [4] work counters: two of the single-step kernel, alternating by step,
     // and two of the two-step kernel, alternating by pair
