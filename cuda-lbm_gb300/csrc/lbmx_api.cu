@@ -187,6 +187,8 @@ static lbmx_status rebuild_pair_lists(lbmx_handle* h, const std::vector<int>& un
     int* at1 = order + nt;
     int* at0 = at1 + nt + 1;
     int k = 0;
+    h->pair_first = 0;
+    for (int t = 0; t < nt; t++) h->pair_first += at[0][(size_t)t + 1] > at[0][(size_t)t] ? 1 : 0;
     for (int pass = 0; pass < 2; pass++)
         for (int t = 0; t < nt; t++)
             if ((at[0][(size_t)t + 1] > at[0][(size_t)t]) == (pass == 0)) order[k++] = t;
@@ -466,6 +468,10 @@ void lbmx::set_step(const lbmx_handle* h, StepArgs& a, long long s) {
     a.tile_chunk = a.parity ? h->tile_chunk : h->tile_chunk0;
     a.special_bits = a.parity ? h->special_bits : h->special_bits0;
     // two work counters, alternating by step: each launch zeroes the other
+    // every other step walks the tiles backwards, and CM_OPT's steps all do,
+    // behind a pre-pass that walks them forwards: a launch starts on what the
+    // one before it touched last, which is still in L2
+    a.reverse = h->p.op == LBMX_CM_OPT || a.parity == 0;
     a.tile_counter = h->tile_counter + (s & 1);
     a.tile_counter_next = h->tile_counter + ((s + 1) & 1);
     // interior store targets: parity 1 -> slot q of the node x + c_q,
@@ -866,12 +872,15 @@ static lbmx_status run_step(lbmx_handle* h, bool store, bool check, bool sums, b
     const bool ext = opt && h->ext_avg;
     h->ext_avg = false;
     const bool lagged = opt && !ext && (h->p.options & LBMX_OPTION_LAGGED_AVERAGES) && h->have_avg;
-    if (opt && !lagged && !ext) {
+    const bool prepass = opt && !lagged && !ext;
+    if (prepass) {
+        // the sums go into the pairs' accumulator sets (CM_OPT steps are
+        // never paired), two in turn
         StepArgs b = a;
-        b.partials = acc;
-        b.counter = h->counter;
-        b.sums = nullptr;
-        b.avg_out = h->avg;
+        b.partials = h->partials + (size_t)(2 + (h->opt_seq & 1)) * kAccPerSet;
+        b.avg_zero = h->partials + (size_t)(2 + ((h->opt_seq + 1) & 1)) * kAccPerSet;
+        h->opt_seq++;
+        a.avg_acc = b.partials;
         LBMX_CUDA(h, dispatch(storage, [&](auto tag) { return launch_opt_prepass<decltype(tag)>(b, st); }));
         h->have_avg = true;
     }
@@ -891,7 +900,8 @@ static lbmx_status run_step(lbmx_handle* h, bool store, bool check, bool sums, b
     a.series = series;
     // with the IBM kernel just launched, the step starts on the items away
     // from the patch while the marker rounds run
-    a.early = h->nm > 0 ? 1 : 0;
+    // (not with a pre-pass between the two, whose averages every node needs)
+    a.early = h->nm > 0 && !prepass ? 1 : 0;
     // the previous step's sums, if it left them to this launch (a pair's two
     // are published by themselves)
     if (h->pend_acc2) {
@@ -931,6 +941,8 @@ static lbmx_status run_pair(lbmx_handle* h, bool store, bool check, bool sums, b
     p.ntiles = h->pair_tiles;
     p.tiles_x = h->pair_tiles_x;
     p.shape = h->pair_shape;
+    p.nfirst = h->pair_first;
+    p.reverse = (int)(h->pair_seq & 1);
     p.num_sms = h->num_sms;
     p.order = h->pair_lists;
     p.sp1_at = p.order + p.ntiles;

@@ -184,6 +184,7 @@ static lbmx_status launch_one(lbmx_batch* b, long long s, int variant) {
     ba.items = b->d_items[parity];
     ba.nitems = b->nitems[parity];
     ba.chunk = b->cfg.chunk;
+    ba.reverse = parity;
     ba.counter = b->counter;
     ba.done = b->done;
     ba.error_word = b->error_word;

@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 && TW * TH > kStageW
                 }
                 break;
             }
-            const int2 it = b.items[item];
+            const int2 it = b.items[b.reverse ? b.nitems - 1 - item : item];
             if (it.y < 0) {
                 // a chunk of special nodes: nothing to stage
                 if (lane == 0) {

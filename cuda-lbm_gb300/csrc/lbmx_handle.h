@@ -85,12 +85,14 @@ struct lbmx_handle {
     CUtensorMap pair_tmap[2];         // descriptors of f and f2 for the two-step tiles
     int* pair_lists = nullptr;        // order, sp1_at, sp0_at, sp1, sp0 (PairArgs) in one buffer
     size_t cap_pair_lists = 0;
-    int pair_tiles = 0, pair_tiles_x = 0, pair_sp1 = 0;  // tiles, tiles per row, entries of sp1
+    int pair_tiles = 0, pair_tiles_x = 0, pair_first = 0;  // tiles, tiles per row, tiles with general-path nodes
+    int pair_sp1 = 0;                 // entries of sp1
     int pair_shape = 0;               // tile shape (lbmx::pair_w, pair_h)
     bool pair_stale = false;          // the lists are still to be built
     bool pair_ready = false;          // the lists match the flags and the lattice's steps can be paired
     bool in_batch = false;            // a batch keeps this lattice's buffer addresses: single steps only
     unsigned long long pair_seq = 0;  // pairs launched
+    unsigned long long opt_seq = 0;   // averages pre-passes left to a step kernel (CM_OPT)
     long long last_step = -2;      // step index of the last single-lattice launch
     double* pend_acc = nullptr;    // accumulators of a step whose sums are not yet published
     double* pend_series = nullptr; // and that step's series entry or null

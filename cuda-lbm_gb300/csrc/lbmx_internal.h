@@ -46,6 +46,10 @@ struct StepArgs {
     double* series;          // or null: the sums' series entry (sums 0..2, then the kinetic
                              // energy when `ke`) is also written here (device-accessible)
     int ke;                  // the sums include the kinetic energy 1/2 rho |u|^2 (accumulator kSumKE)
+    // CM_OPT: the averages pre-pass leaves its sums here for the step kernel,
+    // each CTA of which works the averages out (and writes them to avg)
+    const double* avg_acc;
+    double* avg_zero;        // the pre-pass zeroes this set for the next one
     float* avg_out;          // averages produced by the last block (lagged CM_OPT / pre-pass)
     unsigned int* error_word;// bit 0: non-finite density seen, bit 1: a staging wait gave up
     int check_finite;        // look for non-finite densities this step
@@ -85,6 +89,7 @@ struct StepArgs {
     // (tile_order null: no IBM, tiles in place)
     const int* tile_order;
     int dep_tile;
+    int reverse;                   // tiles from the last to the first (see set_step); no effect with a tile_order
     int early;                     // run the items before the dependent ones before waiting on the preceding grid
     const uint32_t* special_bits;  // 1 bit per unit (see above), or nullptr
     int tiles_x, tiles_y;          // tiles of kStageW x kStageH nodes covering the lattice
@@ -122,6 +127,8 @@ struct PairArgs {
     const float* edge_in;      // a.edge again: the own-node step's old edge-store values
     const int* order;          // [ntiles] tiles in claim order
     int ntiles, tiles_x;
+    int nfirst;                // tiles with general-path nodes: the first of `order`
+    int reverse;               // the tiles behind those from the last to the first
     int shape;                 // tile shape (pair_w, pair_h)
     int num_sms;
     // general-path nodes of each tile t, entries sp[sp_at[t]] .. sp[sp_at[t + 1]]:
@@ -189,6 +196,7 @@ struct BatchArgs {
     const int2* items;            // {lattice, tile >= 0 | -(special chunk + 1)}
     int nitems;
     int chunk;                    // items claimed per atomic
+    int reverse;                  // items from the last to the first
     unsigned long long* counter;  // next item (reset by the last CTA)
     unsigned int* done;           // CTAs finished in this launch
     unsigned int* error_word;     // bit 1: a staging wait gave up

@@ -186,6 +186,46 @@ __device__ __forceinline__ void block_sums(const StepArgs& a, const Acc v[kNumSu
     __threadfence();
 }
 
+// The averages pre-pass' way of leaving its sums to the step kernel behind it:
+// each CTA adds its totals of the three terms with one atomic per sum and is
+// done (publication by the last CTA -- fences, a counter, one more pass over
+// the slots -- took 2 to 3 us of every step).
+__host__ __device__ constexpr int avg_sum(int k) { return k == 0 ? 0 : k + 3; }  // their accumulators
+template <int WARPS>
+__device__ __forceinline__ void leave_averages(double* partials, const Acc v[kNumSums]) {
+    __shared__ Acc sh[WARPS][3];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        Acc t = v[avg_sum(k)];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) sh[warp][k] = t;
+    }
+    __syncthreads();
+    if (tid < 3) {
+        Acc t = 0;
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) t += sh[w][tid];
+        unsigned long long* acc = reinterpret_cast<unsigned long long*>(partials) + (blockIdx.x % kSumSlots) * kNumSums;
+        if (t != 0) atomicAdd(acc + avg_sum(tid), (unsigned long long)t);
+    }
+}
+
+// The averages from such sums, by one warp (the slots are left for the other
+// CTAs to read; the next pre-pass zeroes them).  Every CTA writes the same
+// three values.
+__device__ __forceinline__ void take_averages(const double* acc, float* avg, double n_nodes, int lane) {
+    const unsigned long long* a = reinterpret_cast<const unsigned long long*>(acc) + lane * kNumSums;
+    unsigned long long t[3] = {__ldcg(a + avg_sum(0)), __ldcg(a + avg_sum(1)), __ldcg(a + avg_sum(2))};
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+    const unsigned long long mine = lane == 0 ? t[0] : lane == 1 ? t[1] : t[2];
+    if (lane < 3) avg[lane] = (float)((double)(long long)mine * (1.0 / (double)kFixScale) / n_nodes);
+}
+
 // Post-stream, post-boundary populations of (x, y); returns the node's flag.
 template <typename T>
 __device__ __forceinline__ uint8_t gather_node(const StepArgs& a, int x, int y, float f[9], unsigned* outmask) {
@@ -663,6 +703,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) step_kernel(const StepAr
             // a tile that waits is staged at once all the same: the IBM
             // kernel only reads populations
             if (a.tile_order) tile = __ldg(a.tile_order + tile);
+            else if (a.reverse) tile = ntiles - 1 - tile;
             const int ty = tile / a.tiles_x, tx = tile - ty * a.tiles_x;
             const int x0 = tx * St::TW, y0 = ty * St::TH;
             if (lane == 0) {
@@ -681,6 +722,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) step_kernel(const StepAr
                 mbar_wait(&full[j % St::NST], (unsigned)((j / St::NST) & 1), kWaitLimit);
     } else {
         // consumers
+        if (OP == LBMX_CM_OPT && a.avg_acc) {
+            if (warp == 0) take_averages(a.avg_acc, const_cast<float*>(a.avg), (double)((long long)a.g.nx * a.g.ny), lane);
+            asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory");
+        }
         const int lx = tid % (St::TW / 2), r0 = tid / (St::TW / 2);
         bool waited = !a.early;
         for (int i = 0;; i++) {
@@ -756,60 +801,95 @@ __device__ __forceinline__ void opt_terms(const StepArgs& a, long long off, cons
     v[5] += fix(sqrtf(pxx * pxx + 2.0f * pxy * pxy + pyy * pyy));
 }
 
+// fix() of a pair's sum known to be near `rest`, an even integer: a 32-bit
+// conversion of the difference (exact for t within a factor of two of rest;
+// any t when rest is 0) while that is below one, fix() itself otherwise.
+__device__ __forceinline__ Acc fix_near(float t, float rest) {
+    const float d = t - rest;
+    if (fabsf(d) < 1.0f) return (Acc)__float2int_rn(__fmul_rn(d, kFixScale)) + (Acc)rest * (1ll << 30);
+    return fix(t);
+}
+
 // Grid averages <rho>, <rho |u|>, <|Pi|> of the current step before any
 // collision (update_avg_mag, macroscopics.cuh:50-120), for CM_OPT.  The nodes
 // split as in the step kernel.  Units the tiles take (special bit clear; in a
 // neighbour-access step also off the perimeter) load their 18 populations
-// directly, one unit of two x-neighbours per thread over row segments of
-// 2 * kThreads nodes; the pairs that do not shift in x are single aligned
-// loads.  The parity's general-path units are spread over every thread of
-// the grid, one node each, through the general path.  The terms are summed
-// in exact fixed point, so the averages do not depend on the order.
-template <typename T>
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) opt_prepass_kernel(const StepArgs a) {
+// directly and are worked out in packed arithmetic, the two nodes' terms
+// added before their rounding to fixed point; a warp takes 32 units of one
+// row at a time, its next place found without a division.  The parity's
+// general-path units are spread over every thread of the grid, one node each,
+// through the general path.  The terms are summed in exact fixed point, so
+// the averages do not depend on the order.
+//
+// Instruction issue bounds it (three roots and divisions a node): node by
+// node, with 64-bit addresses, 220 instructions a node took 48.6 us for
+// 4096 x 1024 (151 MB, 22 us at the measured copy rate), 31 to 32 now.
+constexpr int kPrepassThreads = 256, kPrepassCtas = 4;  // (three CTAs per SM: 89 us a step, five spill: 90; four 85)
+template <typename T, int P>
+__global__ void __launch_bounds__(kPrepassThreads, kPrepassCtas) opt_prepass_kernel(const StepArgs a) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" :::);
+    constexpr bool OFS = kOffset<T>;
     Acc v[kNumSums] = {0, 0, 0, 0, 0, 0};
     const Geometry& g = a.g;
     const T* F = static_cast<const T*>(a.f);
-    const int seg_w = 2 * kThreads;
-    const int segs = (g.nx + seg_w - 1) / seg_w;
-    const int items = segs * g.ny;
-    for (int it = blockIdx.x; it < items; it += gridDim.x) {
-        const int y = it / segs;
-        const int x0 = (it - y * segs) * seg_w + 2 * (int)threadIdx.x;
+    // the other set's sums were read by the step before this launch
+    if (a.avg_zero && blockIdx.x == 0 && threadIdx.x < kAccPerSet) a.avg_zero[threadIdx.x] = 0.0;
+    const int lane = threadIdx.x & 31;
+    const int chunks = (g.nx + 63) / 64;  // of 32 units, per row
+    const int nwarps = (int)gridDim.x * (kPrepassThreads / 32);
+    const int first = (int)blockIdx.x * (kPrepassThreads / 32) + (int)(threadIdx.x >> 5);
+    const int dy = nwarps / chunks, dc = nwarps - dy * chunks;
+    int y = first / chunks, c = first - y * chunks;
+    for (; y < g.ny; y += dy, c += dc) {
+        if (c >= chunks) {
+            c -= chunks;
+            if (++y >= g.ny) break;
+        }
+        const int x0 = c * 64 + 2 * lane;
         if (x0 + 1 >= g.nx) continue;  // a lone last node is a general-path unit
-        if (a.parity && !(y > 0 && y < g.ny - 1 && x0 > 0 && x0 + 1 < g.nx - 1)) continue;
-        const long long n0 = (long long)y * g.pitch + x0;
+        if (P && !(y > 0 && y < g.ny - 1 && x0 > 0 && x0 + 1 < g.nx - 1)) continue;
+        const uint32_t n0 = (uint32_t)(y * g.pitch + x0);
         if (a.special_bits) {
-            const long long unit = n0 >> 1;
+            const uint32_t unit = n0 >> 1;
             if ((a.special_bits[unit >> 5] >> (unit & 31)) & 1u) continue;
         }
-        float f0[9], f1[9];
-        const float2 r = Store<T>::ld2(F + a.rest_plane * g.plane + n0, WQ(0));
-        f0[0] = r.x;
-        f1[0] = r.y;
+        V2 f[9];
+        f[0].v = Store<T>::ld2r(F + a.rest_plane * g.plane + n0);
 #pragma unroll
         for (int q = 1; q < 9; q++) {
-            if (!a.parity) {
-                const float2 p = Store<T>::ld2(F + q * g.plane + n0, WQ(q));
-                f0[q] = p.x;
-                f1[q] = p.y;
-            } else if (CX(q) == 0) {
-                const float2 p = Store<T>::ld2(F + OPP(q) * g.plane + n0 - CY(q) * g.pitch, WQ(q));
-                f0[q] = p.x;
-                f1[q] = p.y;
-            } else {
-                const T* src = F + OPP(q) * g.plane + n0 - CY(q) * g.pitch - CX(q);
-                f0[q] = Store<T>::ld(src, WQ(q));
-                f1[q] = Store<T>::ld(src + 1, WQ(q));
-            }
+            const T* src = P ? F + (OPP(q) * g.plane - (CY(q) * g.pitch + CX(q))) : F + q * g.plane;
+            f[q].v = P && CX(q) != 0 ? Store<T>::ld2r_u(src + n0) : Store<T>::ld2r(src + n0);
         }
-        opt_terms(a, n0, f0, v);
-        opt_terms(a, n0 + 1, f1, v);
+        V2 rho = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7])) + f[8];
+        if (OFS) rho = rho + splat(1.0f, rho);  // the weights sum to 1
+        const V2 jx = (f[1] - f[3]) + ((f[5] + f[8]) - (f[6] + f[7]));
+        const V2 jy = (f[2] - f[4]) + ((f[5] + f[6]) - (f[7] + f[8]));
+        V2 Fx = {make_float2(a.body_fx, a.body_fx)}, Fy = {make_float2(a.body_fy, a.body_fy)};
+        if (a.force) {
+            Fx.v = *reinterpret_cast<const float2*>(a.force + n0);
+            Fy.v = *reinterpret_cast<const float2*>(a.force + g.plane + n0);
+        }
+        if (a.ibm_force) {
+            Fx = Fx + V2{__ldcg(reinterpret_cast<const float2*>(a.ibm_force + n0))};
+            Fy = Fy + V2{__ldcg(reinterpret_cast<const float2*>(a.ibm_force + g.plane + n0))};
+        }
+        const V2 inv = vdiv(splat(1.0f, rho), rho);
+        V2 ux = fma(0.5f, Fx, jx) * inv, uy = fma(0.5f, Fy, jy) * inv;
+        if (a.gamma) brinkman<V2>(V2{*reinterpret_cast<const float2*>(a.gamma + n0)}, rho, ux, uy, Fx, Fy);
+        const V2 jm = rho * vsqrt(fma(ux, ux, uy * uy));
+        // offset form: sum c_x^2 w = sum c_y^2 w = 1/3
+        const V2 d = OFS ? (f[5] + f[6]) + ((f[7] + f[8]) + splat(1.0f / 3.0f, rho)) : (f[5] + f[6]) + (f[7] + f[8]);
+        const V2 pxx = (f[1] + f[3]) + d, pyy = (f[2] + f[4]) + d;
+        const V2 pxy = (f[5] + f[7]) - (f[6] + f[8]);
+        const V2 pi = vsqrt(fma(pxx, pxx, fma(2.0f * pxy, pxy, pyy * pyy)));
+        v[0] += fix_near(rho.v.x + rho.v.y, 2.0f);
+        v[4] += fix_near(jm.v.x + jm.v.y, 0.0f);
+        v[5] += fix_near(pi.v.x + pi.v.y, 0.0f);
     }
-    const int nthreads = gridDim.x * kThreads;
-    for (int k = blockIdx.x * kThreads + threadIdx.x; k < 2 * a.nspecial; k += nthreads) {
+    // (from the last thread down: on small lattices the last warps have no units)
+    const int nthreads = gridDim.x * kPrepassThreads;
+    for (int k = nthreads - 1 - (int)(blockIdx.x * kPrepassThreads + threadIdx.x); k < 2 * a.nspecial; k += nthreads) {
         const int off = a.special_units[k >> 1] + (k & 1);
         const int y = off / g.pitch, x = off - y * g.pitch;
         if (x >= g.nx) continue;
@@ -818,7 +898,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) opt_prepass_kernel(const
         gather_node<T>(a, x, y, f, &outmask);
         opt_terms(a, off, f, v);
     }
-    block_sums(a, v, (long long)g.nx * g.ny);
+    if (a.avg_zero) leave_averages<kPrepassThreads / 32>(a.partials, v);
+    else block_sums(a, v, (long long)g.nx * g.ny);
 }
 
 __device__ __forceinline__ void edge_coords(int e, int nx, int ny, int* x, int* y) {
@@ -1080,7 +1161,8 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned 
 
 template <typename T>
 cudaError_t launch_opt_prepass(const StepArgs& a, cudaStream_t s) {
-    return launch_pdl(opt_prepass_kernel<T>, (unsigned)a.num_ctas, kThreads, s, a);
+    return a.parity ? launch_pdl(opt_prepass_kernel<T, 1>, (unsigned)((a.num_ctas * kPrepassCtas + kCtasPerSm - 1) / kCtasPerSm), kPrepassThreads, s, a)
+                    : launch_pdl(opt_prepass_kernel<T, 0>, (unsigned)((a.num_ctas * kPrepassCtas + kCtasPerSm - 1) / kCtasPerSm), kPrepassThreads, s, a);
 }
 
 template <typename T>

@@ -335,7 +335,8 @@ __global__ void __launch_bounds__(kStepThreads, pair_ctas(SHAPE, (int)sizeof(T),
                 }
                 break;
             }
-            const int tile = __ldg(p.order + item);
+            const int tile =
+                __ldg(p.order + (p.reverse && item >= p.nfirst ? p.nfirst + p.ntiles - 1 - item : item));
             const int ty = tile / p.tiles_x, tx = tile - ty * p.tiles_x;
             const int x0 = tx * W, y0 = ty * H;
             const auto publish_slot = [&]() {
