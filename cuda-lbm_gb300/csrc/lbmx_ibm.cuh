@@ -218,7 +218,9 @@ struct IbmFast {
     float2* ft;          // [np] Eulerian force summed over rounds
     float2* mf;          // [nm] marker force of this round
     float2* mt;          // [nm] marker force summed over rounds
-    int2* st;            // [nm * S2] {patch index or -1, weight bits}
+    int2* st;            // [4][nm * S2 / 4] {patch index or -1, weight bits}: stencil point 4 t + p at [p][t],
+                         // so that a warp's threads t read consecutive words (a marker's points side by
+                         // side were 8 shared-memory wavefronts a load instead of 2)
     int2* se;            // [nm * S2] spread entries {marker, weight * ds bits}
     int* sp;             // [np + 1] offsets into se
     int* pn;             // [np] patch node offsets (y * pitch + x)
@@ -249,7 +251,7 @@ __device__ __forceinline__ IbmFast ibm_fast_layout(const IbmData<float>& a, void
 // Stage what does not depend on the flow; no barrier.
 static __device__ void ibm_fast_stage(const IbmData<float>& a, const IbmFast& s, const uint8_t* flags) {
     const int np = a.npatch, nm = a.nm, S2 = a.stencil * a.stencil, nj = nm * S2;
-    for (int j = threadIdx.x; j < nj; j += blockDim.x) s.st[j] = make_int2(a.sten_idx[j], __float_as_int(a.sten_w[j]));
+    for (int j = threadIdx.x; j < nj; j += blockDim.x) s.st[(j & 3) * (nj >> 2) + (j >> 2)] = make_int2(a.sten_idx[j], __float_as_int(a.sten_w[j]));
     const int nsp = a.spread[np];
     for (int i = threadIdx.x; i <= np; i += blockDim.x) s.sp[i] = a.spread[i];
     for (int e = threadIdx.x; e < nsp; e += blockDim.x) {
@@ -281,7 +283,7 @@ __device__ void ibm_fast_iterate_g(const IbmData<float>& a, const IbmFast& s) {
             if (t < nq) {
 #pragma unroll
                 for (int p = 0; p < 4; p++) {
-                    const int2 e = s.st[4 * t + p];
+                    const int2 e = s.st[p * nq + t];
                     if (e.x >= 0) {
                         const float w = __int_as_float(e.y);
                         const float4 q = s.ps[e.x];
