@@ -132,3 +132,28 @@ def test_flags_changed_between_pairs():
         for _ in range(6):
             B.step(1)
         same(A, B)
+
+
+def test_steps_captured_into_a_graph():
+    """Captured steps stay in one buffer, so that a graph can be replayed:
+    six replays of two steps, after steps taken in pairs."""
+    import torch
+    stream = torch.cuda.Stream()
+    c = C.random_state(C.cavity_moving_wall(96, 40, op=C.MRT), seed=6)
+    A = C.make_lattice(c, stream=stream.cuda_stream)
+    B = C.make_lattice(c)
+    A.step(6, flags=0)
+    A.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        A.step(2, flags=0)
+    with torch.cuda.stream(stream):
+        for _ in range(6):
+            graph.replay()
+    A.step(2)  # (moments of the state the replays left)
+    for _ in range(6 + 12 + 2):
+        B.step(1)
+    ra, ua, _ = A.moments()
+    rb, ub, _ = B.moments()
+    np.testing.assert_array_equal(ra, rb)
+    np.testing.assert_array_equal(ua, ub)
