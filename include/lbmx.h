@@ -127,7 +127,9 @@ int32_t lbmx_version(void);
 /* Defaults: BGK, omega 1, FP32, no quirks, 3 IBM iterations, rho_out 1. */
 void lbmx_params_default(lbmx_params* p);
 
-/* Replaces LBM<2>::allocate<S>() + send_consts<S>() (src/core/lbm.cuh:92-125, :63-82). */
+/* Replaces LBM<2>::allocate<S>() + send_consts<S>() (src/core/lbm.cuh:92-125, :63-82).
+ * Allocates a second population buffer, for two steps per launch, while the
+ * device keeps at least half of its memory free beside it. */
 lbmx_status lbmx_create(const lbmx_params* p, lbmx_handle** out);
 
 /* Replaces ~LBM() / LBM::free() (src/core/lbm.cuh:127-140, :379-381). */
@@ -335,7 +337,9 @@ lbmx_status lbmx_moment_sums_noalloc(const float* rho, const float* u, int64_t n
  * force, by a discrete adjoint of the step: forward-mode tangents through the
  * per-node boundary / Brinkman / collision code give each node's Jacobian
  * exactly, and the populations are recomputed from checkpoints taken every
- * `checkpoint_every` steps, so memory is (steps / every + every) states.
+ * `checkpoint_every` steps, so memory is (steps / every + every) states
+ * (the segment's `every` already in the forward run where the device has
+ * them to spare).
  * FP32 populations; any operator; fluid, bounce-back (where it reads no
  * population from outside the domain) and half-way / moving walls; no IBM. */
 typedef struct lbmx_adjoint lbmx_adjoint;
