@@ -203,6 +203,13 @@ __device__ __forceinline__ void adj_avg_terms(const R f[9], R gm, R Fx, R Fy, R 
     out[2] = adj_pimag<R>(f);
 }
 
+// s + e += b exactly but for the addition to e (Knuth's two-sum)
+__device__ __forceinline__ void two_sum(float& s, float& e, float b) {
+    const float t = s + b, bb = t - s;
+    e += (s - (t - bb)) + (b - bb);
+    s = t;
+}
+
 // deterministic block sums of C values; part[block][C] = (or +=) the sum:
 // a fixed shuffle tree within each warp in the values' type (the reverse
 // kernel's per-node gradient terms in FP32: the 64-bit pipe is narrow), the
@@ -257,7 +264,9 @@ __device__ __forceinline__ W2 operator+(W2P a, float b) { return a + W2{both(b)}
 __device__ __forceinline__ W2 operator-(W2 a, W2 b) { return W2{__ffma2_rn(b.v, both(-1.0f), a.v)}; }
 __device__ __forceinline__ W2 operator-(W2 a, W2P b) { return -b + a; }
 __device__ __forceinline__ W2 operator-(W2P a, W2 b) { return a + -b; }
-__device__ __forceinline__ W2 operator-(W2P a, W2P b) { return -b + W2(a); }
+// (the first product is the one kept exact, as in the sum above: it is the
+// larger one where the adjoint of omega depends on it)
+__device__ __forceinline__ W2 operator-(W2P a, W2P b) { return a + W2(-b); }
 __device__ __forceinline__ W2 operator-(W2 a, float b) { return a + -b; }
 __device__ __forceinline__ W2 operator-(float a, W2 b) { return W2{both(a)} - b; }
 __device__ __forceinline__ W2& operator+=(W2& a, W2 b) { return a = a + b; }
@@ -529,13 +538,14 @@ __device__ __forceinline__ void vjp_bgk(const R f[9], R rho, R drho, R ux, R uy,
         const float cx = (float)CX(q), cy = (float)CY(q);
         const R cu = cx * ux + cy * uy;
         const R brm1 = cu * (4.5f * cu + 3.0f) - 1.5f * uu;
-        const R feq = WQ(q) * (rho * brm1 + drho);
+        const R weighed = rho * brm1 + drho;  // feq / w
+        const R noneq = WQ(q) * weighed - f[q];  // feq - f, rounded once: the two are close
         const R gx = 9.0f * cx * cu + 3.0f * (cx - ux);
         const R gy = 9.0f * cy * cu + 3.0f * (cy - uy);
         // fn = f + omega (feq - f) + w pref (gx Fx + gy Fy)
         const R m = mu[q];
         b_f[q] += (1.0f - omega) * m;
-        b_om += (feq - f[q]) * m;
+        b_om += noneq * m;
         b_pref += WQ(q) * (gx * Fx + gy * Fy) * m;
         const R b_gx = WQ(q) * pref * Fx * m, b_gy = WQ(q) * pref * Fy * m;
         b_Fx += WQ(q) * pref * gx * m;
@@ -587,11 +597,15 @@ __device__ __forceinline__ void adj_node_vjp(const AdjArgs& a, const AdjNode* nd
     }
     const R rho = drho + 1.0f;
     const R inv = recip(rho);
-    const R ux0 = (jx + 0.5f * a.fx) * inv, uy0 = (jy + 0.5f * a.fy) * inv;
+    // the quotients by rho with one residual correction (Markstein 1990): the
+    // derivative by omega feels the velocity's last bit
+    const R jfx = jx + 0.5f * a.fx, jfy = jy + 0.5f * a.fy;
+    const R qx = jfx * inv, qy = jfy * inv;
+    const R ux0 = R(jfx - qx * rho) * inv + qx, uy0 = R(jfy - qy * rho) * inv + qy;
     const R sc = recip(R(0.5f * gm + 1.0f));
     const R ux = ux0 * sc, uy = uy0 * sc;
     const R gmr = gm * rho;
-    const R Fx = a.fx - R(gmr * ux), Fy = a.fy - R(gmr * uy);
+    const R Fx = -(gmr * ux) + a.fx, Fy = -(gmr * uy) + a.fy;
     // adjoints
     R b_f[9] = {}, b_S[9] = {};
     R b_rho{}, b_drho{}, b_ux{}, b_uy{}, b_Fx{}, b_Fy{}, b_om{}, b_gm{};
@@ -798,7 +812,7 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjNodes<OP> == 2 ? kAdjReverseBlo
     using R = AdjReal<OP>;
     constexpr int N = kAdjNodes<OP>;
     const long long n = a.g.n;
-    float sums[3] = {0.f, 0.f, 0.f}, asums[3] = {0.f, 0.f, 0.f};
+    float sums[3] = {0.f, 0.f, 0.f}, omega_low = 0.f, asums[3] = {0.f, 0.f, 0.f};
     const uint32_t node0 = blockIdx.x * (N * kAdjBlock) + threadIdx.x;
     if (node0 < n) {
         AdjNode nd[N];
@@ -858,11 +872,32 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjNodes<OP> == 2 ? kAdjReverseBlo
             for (int q = 0; q < 9; q++) (lam_out + q * n)[node] = lane_of(lam[q], h);
             g_gamma[node] = (OP != LBMX_CM ? gg[h] : g_gamma[node]) + (double)lane_of(d_gamma, h);
         }
-        sums[0] = lanes_sum(d_omega);
+        // (the first node's term, then what adding the second's rounded off)
+        sums[0] = lane_of(d_omega, 0);
+        if (N == 2) two_sum(sums[0], omega_low, lane_of(d_omega, N - 1));
         sums[1] = lanes_sum(d_fx);
         sums[2] = lanes_sum(d_fy);
     }
-    adj_block_sum<3, float>(sums, part, true);
+    // The rate's derivative is a sum of terms of both signs, often far below
+    // their magnitudes: its warp sums keep what the additions round off.
+    __shared__ double sh[kAdjBlock / 32][3];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float sb = __shfl_down_sync(0xffffffffu, sums[0], o), eb = __shfl_down_sync(0xffffffffu, omega_low, o);
+        two_sum(sums[0], omega_low, sb);
+        omega_low += eb;
+#pragma unroll
+        for (int k = 1; k < 3; k++) sums[k] += __shfl_down_sync(0xffffffffu, sums[k], o);
+    }
+    if (lane == 0)
+        for (int k = 0; k < 3; k++) sh[warp][k] = (double)sums[k] + (k == 0 ? (double)omega_low : 0.0);
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double t = 0.0;
+        for (int w = 0; w < kAdjBlock / 32; w++) t += sh[w][threadIdx.x];
+        part[(long long)blockIdx.x * 3 + threadIdx.x] += t;
+    }
     if (OP == LBMX_CM_OPT) {
         __syncthreads();
         adj_block_sum<3, float>(asums, avg_part, false);
