@@ -1003,7 +1003,8 @@ struct lbmx_adjoint {
     float* ckpt = nullptr;  // [ncheck - 1][9][n] (the first checkpoint is pc0)
     int ncheck_cap = 0;
     float* seg = nullptr;   // [every - 1][9][n] states after a segment's checkpoint
-    bool kept = false;      // seg holds the last segment of the last forward run
+    bool kept = false;      // seg holds the last segment of the last forward run (until a backward run
+                            // recomputes another segment into it)
     float* lam[2] = {nullptr, nullptr};
     float* avg_hist = nullptr;  // [T + 1][3]
     int avg_cap = 0;
@@ -1377,7 +1378,11 @@ lbmx_status lbmx_adjoint_backward(lbmx_adjoint* a, float* grad_gamma, double* gr
         // recomputed ones (the last segment's may be there from the forward run)
         const float* base = c == 0 ? a->pc0 : a->ckpt + (size_t)(c - 1) * state;
         const auto state_at = [&](int t) { return t == t0 ? base : a->seg + (size_t)(t - t0 - 1) * state; };
-        for (int t = t0 + 1; t < t1 && !(a->kept && c == ncheck - 1); t++) {
+        // the forward run's states are gone once another segment takes their
+        // place: a further backward run recomputes the last one too
+        const bool there = a->kept && c == ncheck - 1;
+        if (c < ncheck - 1) a->kept = false;
+        for (int t = t0 + 1; t < t1 && !there; t++) {
             const float* avg = opt ? a->avg_hist + (size_t)3 * t : nullptr;
             const float* prev = state_at(t - 1);
             float* next = a->seg + (size_t)(t - t0 - 1) * state;

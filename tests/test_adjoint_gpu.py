@@ -151,6 +151,41 @@ def test_checkpoint_interval_leaves_the_gradient_unchanged():
         assert s == out[0][1]
 
 
+@pytest.mark.parametrize("op", [C.BGK, C.CM_OPT])
+@pytest.mark.parametrize("steps,every", [(7, 3), (6, 3), (4, 3), (3, 3), (5, 1)])
+def test_backward_twice_after_one_forward(op, steps, every):
+    """The forward run's kept states serve the first backward run only."""
+    c = case(op)
+    a = make_adjoint(c, every=every)
+    w = np.zeros((3, NY, NX), np.float32)
+    w[1] = 1.0 / NX
+    a.set_objective(w, 1)
+    a.forward(steps)
+    g, s = a.backward()
+    for _ in range(2):
+        g2, s2 = a.backward()
+        np.testing.assert_array_equal(g2, g)
+        assert s2 == s
+    a.forward(steps)  # and a new forward run keeps its own
+    g2, s2 = a.backward()
+    np.testing.assert_array_equal(g2, g)
+    assert s2 == s
+
+
+def test_autograd_retained_graph_gives_the_same_gradient_again():
+    torch = pytest.importorskip("torch")
+    import lbmx_autograd
+    c = case(C.CM)
+    a = make_adjoint(c, every=3)
+    gamma = torch.tensor(c["gamma"], device="cuda", requires_grad=True)
+    J = lbmx_autograd.objective(gamma, torch.tensor(c["omega"]), torch.tensor([1e-5, 0.0]), a, FIRST + 1)
+    J.backward(retain_graph=True)
+    first = gamma.grad.clone()
+    gamma.grad = None
+    J.backward()
+    assert torch.equal(gamma.grad, first)
+
+
 def test_autograd_wrapper_returns_the_adjoint_gradient():
     torch = pytest.importorskip("torch")
     import lbmx_autograd
