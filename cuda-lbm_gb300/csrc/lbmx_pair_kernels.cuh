@@ -111,10 +111,13 @@ __device__ __forceinline__ void unit_sums_add(UnitSums& u, unsigned long long* a
     const int mh = __reduce_add_sync(0xffffffffu, u.m >> 16), ml = __reduce_add_sync(0xffffffffu, u.m & 0xFFFF);
     const int xh = __reduce_add_sync(0xffffffffu, u.x >> 16), xl = __reduce_add_sync(0xffffffffu, u.x & 0xFFFF);
     const int yh = __reduce_add_sync(0xffffffffu, u.y >> 16), yl = __reduce_add_sync(0xffffffffu, u.y & 0xFFFF);
-    // the units' rest mass, 2 * 2^30 each: 2^15 of the high halves
-    const int rest = __reduce_add_sync(0xffffffffu, u.units) << 15;
-    const int hi = lane == 0 ? mh + rest : lane == 1 ? xh : yh, lo = lane == 0 ? ml : lane == 1 ? xl : yl;
-    if (lane < 3) acc[lane] += (unsigned long long)(((Acc)hi << 16) + (Acc)lo);
+    // the units' rest mass, 2 * 2^30 each, in 64 bits: near rest nothing calls
+    // for a warp's total before the end of the launch, and a warp of a large
+    // lattice has more than 2^16 units by then
+    const int units = __reduce_add_sync(0xffffffffu, u.units);
+    const int hi = lane == 0 ? mh : lane == 1 ? xh : yh, lo = lane == 0 ? ml : lane == 1 ? xl : yl;
+    if (lane < 3)
+        acc[lane] += (unsigned long long)(((Acc)hi << 16) + (Acc)lo + (lane == 0 ? (Acc)units << 31 : 0));
     __syncwarp();
     u = UnitSums();
 }

@@ -1,6 +1,8 @@
 """Two steps in one launch against single steps, bit for bit: the pair runs
 the same per-node arithmetic and rounding, so populations, moments and sums
 agree exactly over every boundary, wrap, ragged size and storage it takes."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -117,6 +119,34 @@ def test_series_of_pairs(flags):
         A.step(1, flags=lbmx.STEP_SUMS)
         B.step(1, flags=lbmx.STEP_SUMS)
         np.testing.assert_array_equal(A.moments()[2], B.moments()[2])
+
+
+def test_mass_of_a_large_lattice_near_rest():
+    """More than 2^16 units a warp, none of whose sums calls for a total
+    before the end: 2 CTAs x 8 warps on 152 SMs, FP32 CM."""
+    import torch
+    import lbmx
+    n = 18560
+    free, total = torch.cuda.mem_get_info()
+    if free < 72 * n * n + 30 * n * n + total * 3 // 4:
+        pytest.skip("not enough device memory for a lattice of this size with its second buffer")
+    rho = torch.ones((n, n), device="cuda")
+    u = torch.zeros((2, n, n), device="cuda")
+    torch.cuda.synchronize()
+    L = lbmx.Lattice(n, n, op=lbmx.CM, omega=1.2, periodic=(True, True))
+    sums = []
+    for calls in ([2], [1, 1]):
+        L.init(rho, u)
+        for k in calls:
+            L.step(k)
+        s = (ctypes.c_double * 3)()
+        L._check(L.lib.lbmx_moments(L.h, None, None, s))
+        sums.append(list(s))
+    L.close()
+    del rho, u
+    torch.cuda.empty_cache()
+    assert sums[0] == sums[1]
+    assert abs(sums[0][0] - n * n) < 1e-6 * n * n
 
 
 def test_flags_changed_between_pairs():
