@@ -1004,21 +1004,27 @@ static lbmx_status run_pair(lbmx_handle* h, bool store, bool check, bool sums, b
     return LBMX_OK;
 }
 
-// Whether this call's steps may go in pairs: not into a capture, whose
-// replays would start from the buffer the state was in when it was captured.
+// Whether the handle's stream is being captured into a graph; a handle whose
+// work was ever captured stays with the buffers the graph has the addresses
+// of (can_pair).
+static bool capturing(lbmx_handle* h) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
+    h->captured = h->captured || cs != cudaStreamCaptureStatusNone;
+    return cs != cudaStreamCaptureStatusNone;
+}
+
+// Whether this call's steps may go in pairs: not into a capture, nor after
+// one, since a replay works on the buffers the state was in when it was
+// captured and a pair would leave it in the others.
 // Large 16-bit lattices, where both kernels are bound by instruction issue,
 // keep to single steps when every step reduces sums, which a pair reduces
 // with less occupancy (4096^2 FP16 BGK with sums 126 us a step, 130 in
 // pairs; with the kinetic energy 160 and 183; without sums 111 and 108).
 static bool can_pair(lbmx_handle* h, bool every_step_sums) {
+    if (capturing(h) || h->captured) return false;
     if (!(h->pair_ready || h->pair_stale) || h->in_batch || h->nm > 0) return false;
     if (every_step_sums && h->pair_shape == 0 && elem_size(h->p.storage) == 2) return false;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    if (cs != cudaStreamCaptureStatusNone) return false;
     return !h->pair_stale || (rebuild_special(h) == LBMX_OK && h->pair_ready);
 }
 
@@ -1080,7 +1086,7 @@ lbmx_status lbmx_step_sums(lbmx_handle* h, int32_t nsteps, uint32_t flags, doubl
     // a step's entry: {rho, rho ux, rho uy}, then the kinetic energy
     const bool ke = (flags & LBMX_STEP_KINETIC_ENERGY) != 0;
     const size_t stride = ke ? 4 : 3;
-    const bool pairs = direct && can_pair(h, true);
+    const bool pairs = can_pair(h, true) && direct;
     for (int i = 0; i < nsteps; i++) {
         if (pairs && !(h->t & 1) && nsteps - i >= 2) {
             const bool ends = i + 2 == nsteps;
@@ -1120,6 +1126,7 @@ lbmx_status lbmx_step_forces(lbmx_handle* h, int32_t nsteps, uint32_t flags, dou
     if (nsteps < 0) return fail(h, LBMX_ERR_INVALID_ARGUMENT, "lbmx_step_forces: nsteps < 0");
     if (h->nm <= 0) return fail(h, LBMX_ERR_INVALID_ARGUMENT, "lbmx_step_forces: the lattice has no IBM markers");
     cudaSetDevice(h->p.device);
+    capturing(h);
     const bool check = (flags & LBMX_STEP_CHECK_FINITE) != 0;
     if (check) LBMX_CUDA(h, cudaMemsetAsync(h->error_word, 0, sizeof(unsigned int), h->stream));
     // as lbmx_step_sums: written by the kernel where it can reach the series,
@@ -1261,6 +1268,7 @@ static lbmx_status halo_copy(lbmx_handle* h, int32_t row, uint32_t plane_mask, v
     if (row < 0 || row >= h->g.ny || plane_mask == 0 || plane_mask > 0x1FFu)
         return fail(h, LBMX_ERR_INVALID_ARGUMENT, "%s: row %d or plane mask 0x%x out of range", who, row, plane_mask);
     cudaSetDevice(h->p.device);
+    capturing(h);
     const size_t es = elem_size(h->p.storage), bytes = (size_t)h->g.nx * es;
     char* f = static_cast<char*>(h->f);
     char* b = static_cast<char*>(buf);

@@ -154,7 +154,13 @@ lbmx_status lbmx_set_force_field(lbmx_handle* h, const float* force);
 
 /* Replaces one pass of the reference loop body (src/main.cu:96-114):
  * stream, boundaries, macroscopics, IBM, force correction, averages,
- * equilibrium and collision, fused.  Stores moments on the last step. */
+ * equilibrium and collision, fused.  Stores moments on the last step.
+ * Calls on a stream that is being captured go into the graph.  Each replay
+ * advances the lattice's state by the captured steps: capture an even number
+ * of them and replay from an even step.  lbmx_time counts the captured steps
+ * once, when they are captured.  Direct steps and lbmx_init_from_fields may
+ * stand between replays: after its first capture a lattice takes all its
+ * steps one per launch, in the buffers the graph works on. */
 lbmx_status lbmx_step(lbmx_handle* h, int32_t nsteps);
 lbmx_status lbmx_step_ex(lbmx_handle* h, int32_t nsteps, uint32_t flags);
 

@@ -187,3 +187,41 @@ def test_steps_captured_into_a_graph():
     rb, ub, _ = B.moments()
     np.testing.assert_array_equal(ra, rb)
     np.testing.assert_array_equal(ua, ub)
+
+
+def test_direct_steps_between_replays():
+    """After a capture the state stays in the graph's buffers: replays and
+    direct steps in turn, then a fresh state."""
+    import torch
+    stream = torch.cuda.Stream()
+    c = C.random_state(C.cavity_moving_wall(96, 40, op=C.MRT), seed=6)
+    A = C.make_lattice(c, stream=stream.cuda_stream)
+    B = C.make_lattice(c)
+    A.step(2, flags=0)
+    A.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        A.step(2, flags=0)
+
+    def replay(n):
+        with torch.cuda.stream(stream):
+            for _ in range(n):
+                graph.replay()
+
+    def check(steps):
+        for _ in range(steps):
+            B.step(1)
+        for x, y in zip(A.moments(), B.moments()):
+            np.testing.assert_array_equal(x, y)
+
+    replay(3)
+    A.step(2)
+    check(2 + 6 + 2)
+    replay(1)
+    A.step(4)
+    check(2 + 4)
+    for L in (A, B):
+        L.init(np.asarray(c["rho"], np.float32), np.asarray(c["u"], np.float32))
+    replay(2)
+    A.step(2)
+    check(4 + 2)
