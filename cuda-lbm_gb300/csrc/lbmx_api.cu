@@ -875,12 +875,20 @@ static lbmx_status run_step(lbmx_handle* h, bool store, bool check, bool sums, b
     const bool prepass = opt && !lagged && !ext;
     if (prepass) {
         // the sums go into the pairs' accumulator sets (CM_OPT steps are
-        // never paired), two in turn
+        // never paired), two in turn; in a captured step, whose replays need
+        // not take turns, the pre-pass publishes the averages itself and
+        // leaves its set zero
         StepArgs b = a;
-        b.partials = h->partials + (size_t)(2 + (h->opt_seq & 1)) * kAccPerSet;
-        b.avg_zero = h->partials + (size_t)(2 + ((h->opt_seq + 1) & 1)) * kAccPerSet;
-        h->opt_seq++;
-        a.avg_acc = b.partials;
+        if (h->capture_now) {
+            b.partials = acc;
+            b.counter = h->counter;
+            b.avg_out = h->avg;
+        } else {
+            b.partials = h->partials + (size_t)(2 + (h->opt_seq & 1)) * kAccPerSet;
+            b.avg_zero = h->partials + (size_t)(2 + ((h->opt_seq + 1) & 1)) * kAccPerSet;
+            h->opt_seq++;
+            a.avg_acc = b.partials;
+        }
         LBMX_CUDA(h, dispatch(storage, [&](auto tag) { return launch_opt_prepass<decltype(tag)>(b, st); }));
         h->have_avg = true;
     }
@@ -1010,8 +1018,9 @@ static lbmx_status run_pair(lbmx_handle* h, bool store, bool check, bool sums, b
 static bool capturing(lbmx_handle* h) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
-    h->captured = h->captured || cs != cudaStreamCaptureStatusNone;
-    return cs != cudaStreamCaptureStatusNone;
+    h->capture_now = cs != cudaStreamCaptureStatusNone;
+    h->captured = h->captured || h->capture_now;
+    return h->capture_now;
 }
 
 // Whether this call's steps may go in pairs: not into a capture, nor after

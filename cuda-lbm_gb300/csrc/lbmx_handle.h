@@ -91,6 +91,7 @@ struct lbmx_handle {
     bool pair_stale = false;          // the lists are still to be built
     bool pair_ready = false;          // the lists match the flags and the lattice's steps can be paired
     bool in_batch = false;            // a batch keeps this lattice's buffer addresses: single steps only
+    bool capture_now = false;         // the running call's steps go into a graph
     bool captured = false;            // work of this handle was captured into a graph: single steps from then on
     unsigned long long pair_seq = 0;  // pairs launched
     unsigned long long opt_seq = 0;   // averages pre-passes left to a step kernel (CM_OPT)

@@ -225,3 +225,31 @@ def test_direct_steps_between_replays():
     replay(2)
     A.step(2)
     check(4 + 2)
+
+
+def test_captured_averages_pre_pass_replayed_alone():
+    """CM_OPT with lagged averages: only the first of the two captured steps
+    has a pre-pass, and each of its replays computes the same averages as a
+    direct step from that state."""
+    import torch
+    import lbmx
+    stream = torch.cuda.Stream()
+    c = C.random_state(C.cavity_moving_wall(96, 40, op=C.CM_OPT), seed=8)
+    A = C.make_lattice(c, options=lbmx.OPTION_LAGGED_AVERAGES, stream=stream.cuda_stream)
+    B = C.make_lattice(c)
+    first, second = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    for graph in (first, second):
+        with torch.cuda.graph(graph, stream=stream):
+            A.step(1)
+    for _ in range(3):
+        with torch.cuda.stream(stream):
+            first.replay()
+        B.step(1)
+        avg = B.averages()
+        np.testing.assert_allclose(A.averages(), avg, rtol=1e-6)
+        with torch.cuda.stream(stream):
+            second.replay()
+        B.set_averages(avg)  # the second step lags: the averages of the first
+        B.step(1)
+        for x, y in zip(A.moments(), B.moments()):
+            np.testing.assert_allclose(x, y, rtol=1e-6, atol=1e-6)
