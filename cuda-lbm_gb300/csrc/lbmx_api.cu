@@ -1032,7 +1032,7 @@ static bool capturing(lbmx_handle* h) {
 // pairs; with the kinetic energy 160 and 183; without sums 111 and 108).
 static bool can_pair(lbmx_handle* h, bool every_step_sums) {
     if (capturing(h) || h->captured) return false;
-    if (!(h->pair_ready || h->pair_stale) || h->in_batch || h->nm > 0) return false;
+    if (!(h->pair_ready || h->pair_stale) || h->batches->load() > 0 || h->nm > 0) return false;
     if (every_step_sums && h->pair_shape == 0 && elem_size(h->p.storage) == 2) return false;
     return !h->pair_stale || (rebuild_special(h) == LBMX_OK && h->pair_ready);
 }

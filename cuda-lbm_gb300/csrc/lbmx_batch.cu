@@ -23,6 +23,7 @@ constexpr int kVariants = 3;
 
 struct lbmx_batch {
     std::vector<lbmx_handle*> lat;
+    std::vector<std::shared_ptr<std::atomic<int>>> memberships;  // the lattices' counts of batches
     int device = 0, storage = 0, op = 0, num_sms = 1;
     cudaStream_t stream = nullptr;
     bool own_stream = false;  // false: every lattice runs on this one stream
@@ -300,6 +301,7 @@ void lbmx_batch_destroy(lbmx_batch* b) {
     // wait for the device instead of touching it
     if (b->own_stream && b->stream) cudaStreamSynchronize(b->stream);
     else cudaDeviceSynchronize();
+    for (const auto& m : b->memberships) --*m;
     drop_graphs(b);
     cudaFree(b->d_args); cudaFree(b->d_tmaps); cudaFree(b->d_items[0]); cudaFree(b->d_items[1]);
     cudaFree(b->counter); cudaFree(b->done); cudaFree(b->error_word); cudaFree(b->step);
@@ -375,7 +377,10 @@ lbmx_status lbmx_batch_create(lbmx_handle* const* lattices, int32_t count, lbmx_
     cudaMemsetAsync(b->done, 0, sizeof(unsigned int), b->stream);
     cudaMemsetAsync(b->error_word, 0, sizeof(unsigned int), b->stream);
     if (refresh(b) != LBMX_OK) return cleanup(LBMX_ERR_CUDA, b->err);
-    for (lbmx_handle* h : b->lat) h->in_batch = true;
+    for (lbmx_handle* h : b->lat) {
+        b->memberships.push_back(h->batches);
+        ++*h->batches;
+    }
     *out = b;
     return LBMX_OK;
 }

@@ -4,6 +4,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <atomic>
+#include <memory>
 #include <vector>
 
 #include "lbmx.h"
@@ -90,7 +92,10 @@ struct lbmx_handle {
     int pair_shape = 0;               // tile shape (lbmx::pair_w, pair_h)
     bool pair_stale = false;          // the lists are still to be built
     bool pair_ready = false;          // the lists match the flags and the lattice's steps can be paired
-    bool in_batch = false;            // a batch keeps this lattice's buffer addresses: single steps only
+    // batches this lattice is in: single steps meanwhile, since a batch keeps
+    // its buffers' addresses in device arguments and graphs, rebuilt (with a
+    // wait) when they change.  Shared with the batches, which may outlive it.
+    std::shared_ptr<std::atomic<int>> batches = std::make_shared<std::atomic<int>>(0);
     bool capture_now = false;         // the running call's steps go into a graph
     bool captured = false;            // work of this handle was captured into a graph: single steps from then on
     unsigned long long pair_seq = 0;  // pairs launched
