@@ -986,7 +986,15 @@ __global__ void adj_to_float_kernel(const double* src, float* dst, long long n) 
 
 using namespace lbmx;
 
-struct lbmx_adjoint {
+struct lbmx_adjoint : Spare {
+    // the kept segment, with no call running: a backward run recomputes it
+    bool give_back() override {
+        if (!seg) return false;
+        cudaFree(seg);
+        seg = nullptr;
+        kept = false;
+        return true;
+    }
     lbmx_params p;
     AdjArgs args;
     cudaStream_t stream = nullptr;
@@ -1147,6 +1155,7 @@ void lbmx_adjoint_destroy(lbmx_adjoint* a) {
     cudaGetDevice(&cur);
     cudaSetDevice(a->p.device);
     if (a->stream) cudaStreamSynchronize(a->stream);
+    spare_remove(a);
     cudaFree(a->flags); cudaFree(a->gamma); cudaFree(a->weights); cudaFree(a->pc0);
     cudaFree(a->ping[0]); cudaFree(a->ping[1]); cudaFree(a->ckpt); cudaFree(a->seg);
     cudaFree(a->lam[0]); cudaFree(a->lam[1]); cudaFree(a->avg_hist); cudaFree(a->jnode);
@@ -1206,15 +1215,15 @@ lbmx_status lbmx_adjoint_create(const lbmx_params* p, const uint8_t* flags, int3
         return LBMX_ERR_OUT_OF_MEMORY;
     };
     const size_t state = (size_t)9 * a->n * sizeof(float);
-    if (cudaMalloc((void**)&a->flags, (size_t)a->n) != cudaSuccess ||
-        cudaMalloc((void**)&a->pc0, state) != cudaSuccess || cudaMalloc((void**)&a->ping[0], state) != cudaSuccess ||
-        cudaMalloc((void**)&a->ping[1], state) != cudaSuccess ||
-        cudaMalloc((void**)&a->jnode, (size_t)a->n * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void**)&a->part, (size_t)a->blocks * 3 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void**)&a->avg_part, (size_t)a->blocks * 3 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void**)&a->red, (8 + 3 * kSumBlocks) * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void**)&a->rho_out, (size_t)a->n * sizeof(float)) != cudaSuccess ||
-        cudaMalloc((void**)&a->u_out, (size_t)2 * a->n * sizeof(float)) != cudaSuccess)
+    if (device_alloc(&a->flags, (size_t)a->n) != cudaSuccess ||
+        device_alloc(&a->pc0, state) != cudaSuccess || device_alloc(&a->ping[0], state) != cudaSuccess ||
+        device_alloc(&a->ping[1], state) != cudaSuccess ||
+        device_alloc(&a->jnode, (size_t)a->n * sizeof(double)) != cudaSuccess ||
+        device_alloc(&a->part, (size_t)a->blocks * 3 * sizeof(double)) != cudaSuccess ||
+        device_alloc(&a->avg_part, (size_t)a->blocks * 3 * sizeof(double)) != cudaSuccess ||
+        device_alloc(&a->red, (8 + 3 * kSumBlocks) * sizeof(double)) != cudaSuccess ||
+        device_alloc(&a->rho_out, (size_t)a->n * sizeof(float)) != cudaSuccess ||
+        device_alloc(&a->u_out, (size_t)2 * a->n * sizeof(float)) != cudaSuccess)
         return bail("cudaMalloc failed");
     a->sum_part = a->red + 8;
     if (p->stream) {
@@ -1225,6 +1234,8 @@ lbmx_status lbmx_adjoint_create(const lbmx_params* p, const uint8_t* flags, int3
     }
     cudaMemcpy(a->flags, fl.data(), fl.size(), cudaMemcpyHostToDevice);
     a->args.flags = a->flags;
+    a->device = p->device;
+    spare_add(a);
     *out = a;
     return LBMX_OK;
 }
@@ -1233,7 +1244,7 @@ lbmx_status lbmx_adjoint_set_state(lbmx_adjoint* a, const float* rho, const floa
     if (!a || !rho || !u) return afail(a, LBMX_ERR_INVALID_ARGUMENT, "lbmx_adjoint_set_state: NULL argument");
     cudaSetDevice(a->p.device);
     float* tmp = nullptr;
-    ADJ_CUDA(a, cudaMalloc((void**)&tmp, (size_t)3 * a->n * sizeof(float)));
+    ADJ_CUDA(a, device_alloc(&tmp, (size_t)3 * a->n * sizeof(float)));
     cudaMemcpyAsync(tmp, rho, (size_t)a->n * sizeof(float), cudaMemcpyDefault, a->stream);
     cudaMemcpyAsync(tmp + a->n, u, (size_t)2 * a->n * sizeof(float), cudaMemcpyDefault, a->stream);
     adj_init_kernel<<<grid_of(a->n), kAdjBlock, 0, a->stream>>>(a->args.g, tmp, tmp + a->n, a->pc0);
@@ -1252,7 +1263,7 @@ lbmx_status lbmx_adjoint_set_gamma(lbmx_adjoint* a, const float* gamma) {
         cudaFree(a->gamma);
         a->gamma = nullptr;
     } else {
-        if (!a->gamma) ADJ_CUDA(a, cudaMalloc((void**)&a->gamma, (size_t)a->n * sizeof(float)));
+        if (!a->gamma) ADJ_CUDA(a, device_alloc(&a->gamma, (size_t)a->n * sizeof(float)));
         ADJ_CUDA(a, cudaMemcpyAsync(a->gamma, gamma, (size_t)a->n * sizeof(float), cudaMemcpyDefault, a->stream));
         ADJ_CUDA(a, cudaStreamSynchronize(a->stream));
     }
@@ -1276,7 +1287,7 @@ lbmx_status lbmx_adjoint_set_objective(lbmx_adjoint* a, const float* weights, in
     if (!a || !weights) return afail(a, LBMX_ERR_INVALID_ARGUMENT, "lbmx_adjoint_set_objective: NULL argument");
     if (first_step < 1) return afail(a, LBMX_ERR_INVALID_ARGUMENT, "lbmx_adjoint_set_objective: first_step < 1");
     cudaSetDevice(a->p.device);
-    if (!a->weights) ADJ_CUDA(a, cudaMalloc((void**)&a->weights, (size_t)3 * a->n * sizeof(float)));
+    if (!a->weights) ADJ_CUDA(a, device_alloc(&a->weights, (size_t)3 * a->n * sizeof(float)));
     ADJ_CUDA(a, cudaMemcpyAsync(a->weights, weights, (size_t)3 * a->n * sizeof(float), cudaMemcpyDefault, a->stream));
     ADJ_CUDA(a, cudaStreamSynchronize(a->stream));
     a->args.weights = a->weights;
@@ -1307,20 +1318,21 @@ lbmx_status lbmx_adjoint_forward(lbmx_adjoint* a, int32_t nsteps, double* object
     if (ncheck > a->ncheck_cap) {
         cudaFree(a->ckpt);
         a->ckpt = nullptr;
-        if (ncheck > 1) ADJ_CUDA(a, cudaMalloc((void**)&a->ckpt, (size_t)(ncheck - 1) * state * sizeof(float)));
+        if (ncheck > 1) ADJ_CUDA(a, device_alloc(&a->ckpt, (size_t)(ncheck - 1) * state * sizeof(float)));
         a->ncheck_cap = ncheck;
     }
     if (nsteps + 1 > a->avg_cap) {
         cudaFree(a->avg_hist);
         a->avg_hist = nullptr;
-        ADJ_CUDA(a, cudaMalloc((void**)&a->avg_hist, (size_t)3 * (nsteps + 1) * sizeof(float)));
+        ADJ_CUDA(a, device_alloc(&a->avg_hist, (size_t)3 * (nsteps + 1) * sizeof(float)));
         a->avg_cap = nsteps + 1;
     }
     // The last segment's states stay in the segment buffer the backward run
     // would recompute them into, where that buffer is there or the device
     // has room for it to spare (a run that never goes backward needs none).
+    SpareUse use(*a);
     const size_t seg_bytes = (size_t)(a->every - 1) * state * sizeof(float);
-    if (!a->seg && seg_bytes) {
+    if (!a->seg && seg_bytes && !(a->p.options & LBMX_OPTION_SINGLE_BUFFER)) {
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < seg_bytes + total_b / 2 ||
             cudaMalloc((void**)&a->seg, seg_bytes) != cudaSuccess)
@@ -1357,14 +1369,15 @@ lbmx_status lbmx_adjoint_backward(lbmx_adjoint* a, float* grad_gamma, double* gr
     if (!a->have_forward)
         return afail(a, LBMX_ERR_NOT_INITIALIZED, "lbmx_adjoint_backward: run lbmx_adjoint_forward with these inputs first");
     cudaSetDevice(a->p.device);
+    SpareUse use(*a);
     const size_t state = (size_t)9 * a->n;
     if (!a->seg && a->every > 1)
-        ADJ_CUDA(a, cudaMalloc((void**)&a->seg, (size_t)(a->every - 1) * state * sizeof(float)));
+        ADJ_CUDA(a, device_alloc(&a->seg, (size_t)(a->every - 1) * state * sizeof(float)));
     if (!a->lam[0]) {
-        ADJ_CUDA(a, cudaMalloc((void**)&a->lam[0], state * sizeof(float)));
-        ADJ_CUDA(a, cudaMalloc((void**)&a->lam[1], state * sizeof(float)));
+        ADJ_CUDA(a, device_alloc(&a->lam[0], state * sizeof(float)));
+        ADJ_CUDA(a, device_alloc(&a->lam[1], state * sizeof(float)));
     }
-    if (!a->g_gamma) ADJ_CUDA(a, cudaMalloc((void**)&a->g_gamma, (size_t)a->n * sizeof(double)));
+    if (!a->g_gamma) ADJ_CUDA(a, device_alloc(&a->g_gamma, (size_t)a->n * sizeof(double)));
     ADJ_CUDA(a, cudaMemsetAsync(a->g_gamma, 0, (size_t)a->n * sizeof(double), a->stream));
     ADJ_CUDA(a, cudaMemsetAsync(a->part, 0, (size_t)a->blocks * 3 * sizeof(double), a->stream));
     const bool opt = a->p.op == LBMX_CM_OPT;

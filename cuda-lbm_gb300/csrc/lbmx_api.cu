@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <algorithm>
@@ -38,6 +39,48 @@ static lbmx_status fail(lbmx_handle* h, lbmx_status code, const char* fmt, ...) 
             return fail((h), e_ == cudaErrorMemoryAllocation ? LBMX_ERR_OUT_OF_MEMORY : LBMX_ERR_CUDA, \
                         "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__);        \
     } while (0)
+
+static std::mutex g_spares_lock;
+static std::vector<Spare*>& g_spares = *new std::vector<Spare*>;  // outlives any static handle of the caller's
+
+void lbmx::spare_add(Spare* s) {
+    std::lock_guard<std::mutex> l(g_spares_lock);
+    g_spares.push_back(s);
+}
+
+void lbmx::spare_remove(Spare* s) {
+    std::lock_guard<std::mutex> l(g_spares_lock);
+    g_spares.erase(std::remove(g_spares.begin(), g_spares.end(), s), g_spares.end());
+}
+
+cudaError_t lbmx::device_alloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> l(g_spares_lock);
+    for (Spare* s : g_spares) {
+        cudaGetLastError();
+        // (one in use, be it by this thread, is not waited for)
+        if (s->device != dev || s->busy.exchange(true)) continue;
+        const bool freed = s->give_back();
+        s->busy = false;
+        if (freed && (e = cudaMalloc(p, bytes)) != cudaErrorMemoryAllocation) return e;
+    }
+    return e;
+}
+
+// The second population buffer; the init fields' staging gets its own
+// memory, as in a lattice without one.  cudaFree waits for the device.
+bool lbmx_handle::give_back() {
+    if (!f2) return false;
+    pair_ready = pair_stale = false;
+    cudaFree(f2_alloc);
+    f2 = f2_alloc = nullptr;
+    staging = nullptr;
+    if (cudaMalloc((void**)&staging, (size_t)3 * g.nx * g.ny * sizeof(float)) != cudaSuccess) cudaGetLastError();
+    return true;
+}
 
 size_t lbmx::elem_size(int storage) { return storage == LBMX_STORAGE_F32 ? 4 : 2; }
 
@@ -122,7 +165,7 @@ static cudaError_t upload_list(const void* src, size_t bytes, void** buf, size_t
         cudaFree(*buf);
         *buf = nullptr;
         *cap = 0;
-        const cudaError_t e = cudaMalloc(buf, std::max<size_t>(bytes, 4));
+        const cudaError_t e = device_alloc(buf, std::max<size_t>(bytes, 4));
         if (e != cudaSuccess) return e;
         *cap = std::max<size_t>(bytes, 4);
     }
@@ -201,7 +244,10 @@ static lbmx_status rebuild_pair_lists(lbmx_handle* h, const std::vector<int>& un
         sp += found[step].size();
     }
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
-    LBMX_CUDA(h, upload_list(all.data(), all.size() * sizeof(int), (void**)&h->pair_lists, &h->cap_pair_lists));
+    if (upload_list(all.data(), all.size() * sizeof(int), (void**)&h->pair_lists, &h->cap_pair_lists) != cudaSuccess) {
+        cudaGetLastError();  // no room for them: single steps
+        return LBMX_OK;
+    }
     h->pair_tiles = nt;
     h->pair_tiles_x = tx;
     h->pair_sp1 = (int)n1;
@@ -368,7 +414,7 @@ static lbmx_status rebuild_special(lbmx_handle* h, bool pair_lists = true) {
         }
         h->dep_tile = (int)first.size();
         first.insert(first.end(), last.begin(), last.end());
-        LBMX_CUDA(h, cudaMalloc((void**)&h->tile_order, first.size() * sizeof(int)));
+        LBMX_CUDA(h, device_alloc(&h->tile_order, first.size() * sizeof(int)));
         LBMX_CUDA(h, cudaMemcpy(h->tile_order, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
     }
     // Persistent CTAs walk the work list, kCtasPerSm per SM, except in the
@@ -529,8 +575,9 @@ void lbmx_destroy(lbmx_handle* h) {
     cudaSetDevice(h->p.device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     free_ibm(h);
+    spare_remove(h);
     if (h->staging != h->f2) cudaFree(h->staging);
-    cudaFree(h->f_alloc); cudaFree(h->edge_alloc); cudaFree(h->words); cudaFree(h->pair_lists); cudaFree(h->flags);
+    cudaFree(h->f_alloc); cudaFree(h->f2_alloc); cudaFree(h->edge_alloc); cudaFree(h->words); cudaFree(h->pair_lists); cudaFree(h->flags);
     cudaFree(h->force); cudaFree(h->gamma); cudaFree(h->rho_out); cudaFree(h->pop_out); cudaFree(h->raw_sums);
     cudaFree(h->special_units); cudaFree(h->bits_buf); cudaFree(h->special_units0); cudaFree(h->bits0_buf);
     cudaFree(h->tile_order);
@@ -575,7 +622,7 @@ lbmx_status lbmx_create(const lbmx_params* p, lbmx_handle** out) {
     const long long n = (long long)g.nx * g.ny;
 #define ALLOC(ptr, bytes)                                                                  \
     do {                                                                                    \
-        cudaError_t e_ = cudaMalloc((void**)&(ptr), (bytes));                               \
+        cudaError_t e_ = device_alloc(&(ptr), (bytes));                                     \
         if (e_ != cudaSuccess) {                                                            \
             fail(nullptr, LBMX_ERR_OUT_OF_MEMORY, "lbmx_create: cudaMalloc(%zu): %s",       \
                  (size_t)(bytes), cudaGetErrorString(e_));                                  \
@@ -587,21 +634,21 @@ lbmx_status lbmx_create(const lbmx_params* p, lbmx_handle** out) {
     if (h->num_sms < 1) h->num_sms = 1;
     // The populations, and the second population buffer of the two-step
     // launches while the device keeps at least half of its memory free beside
-    // it (a spare that lattices created later may need instead).  It holds
-    // the init fields too: nothing else is in it between launches.
+    // it (given back to later allocations that need it, Spare).  It holds the
+    // init fields too: nothing else is in it between launches.
     const int es = (int)elem_size(p->storage);
     const size_t f_bytes = (((size_t)h->nplanes * g.plane + 2 * kGuardElems) * es + 255) / 256 * 256;
+    h->device = p->device;
+    ALLOC(h->f_alloc, f_bytes);
     size_t free_b = 0, total_b = 0;
     const bool pairs = p->op != LBMX_CM_OPT && !(p->quirks & LBMX_QUIRK_REST_LAG) &&
+                       !(p->options & LBMX_OPTION_SINGLE_BUFFER) &&
                        (unsigned long long)g.plane * es <= 0xFFFFFFFFull &&
-                       cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b >= 2 * f_bytes + total_b / 2 &&
-                       cudaMalloc(&h->f_alloc, 2 * f_bytes) == cudaSuccess;
-    if (!pairs) {
-        cudaGetLastError();
-        ALLOC(h->f_alloc, f_bytes);
-    }
+                       cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b >= f_bytes + total_b / 2 &&
+                       cudaMalloc(&h->f2_alloc, f_bytes) == cudaSuccess;
+    if (!pairs) cudaGetLastError();
     h->f = static_cast<char*>(h->f_alloc) + (size_t)kGuardElems * es;
-    if (pairs) h->f2 = static_cast<char*>(h->f) + f_bytes;
+    if (pairs) h->f2 = static_cast<char*>(h->f2_alloc) + (size_t)kGuardElems * es;
     h->pair_shape = pair_shape(g.nx, g.ny, es, p->op, h->num_sms);
     const int tw = step_tile_w(es), th = step_tile_h(es), pw = pair_w(h->pair_shape), ph = pair_h(h->pair_shape, es) + 2;
     bool maps = encode_population_map(h, &h->tmap, tw, th);
@@ -663,6 +710,7 @@ lbmx_status lbmx_create(const lbmx_params* p, lbmx_handle** out) {
         lbmx_destroy(h);
         return LBMX_ERR_OUT_OF_MEMORY;
     }
+    if (h->f2) spare_add(h);
     *out = h;
     return LBMX_OK;
 }
@@ -724,7 +772,7 @@ lbmx_status lbmx_set_flags(lbmx_handle* h, const uint8_t* flags) {
         return rebuild_special(h);
     }
     if (!h->flags) {
-        cudaError_t e = cudaMalloc((void**)&h->flags, (size_t)g.plane);
+        cudaError_t e = device_alloc(&h->flags, (size_t)g.plane);
         if (e != cudaSuccess) return fail(h, LBMX_ERR_OUT_OF_MEMORY, "lbmx_set_flags: cudaMalloc failed");
     }
     h->flags_host.assign((size_t)g.plane, 0);
@@ -758,7 +806,7 @@ static lbmx_status upload_force(lbmx_handle* h, const float* force) {
         return LBMX_OK;
     }
     if (!h->force) {
-        cudaError_t e = cudaMalloc((void**)&h->force, (size_t)2 * g.plane * sizeof(float));
+        cudaError_t e = device_alloc(&h->force, (size_t)2 * g.plane * sizeof(float));
         if (e != cudaSuccess) return fail(h, LBMX_ERR_OUT_OF_MEMORY, "force field: cudaMalloc failed");
     }
     LBMX_CUDA(h, cudaMemsetAsync(h->force, 0, (size_t)2 * g.plane * sizeof(float), h->stream));
@@ -781,7 +829,7 @@ lbmx_status lbmx_set_brinkman(lbmx_handle* h, const float* gamma) {
         return LBMX_OK;
     }
     if (!h->gamma) {
-        cudaError_t e = cudaMalloc((void**)&h->gamma, (size_t)g.plane * sizeof(float));
+        cudaError_t e = device_alloc(&h->gamma, (size_t)g.plane * sizeof(float));
         if (e != cudaSuccess) return fail(h, LBMX_ERR_OUT_OF_MEMORY, "lbmx_set_brinkman: cudaMalloc failed");
         LBMX_CUDA(h, cudaMemsetAsync(h->gamma, 0, (size_t)g.plane * sizeof(float), h->stream));
     }
@@ -802,12 +850,14 @@ lbmx_status lbmx_init_from_fields(lbmx_handle* h, const float* rho, const float*
     cudaSetDevice(h->p.device);
     const Geometry& g = h->g;
     const long long n = (long long)g.nx * g.ny;
-    LBMX_CUDA(h, cudaMemcpyAsync(h->staging, rho, n * sizeof(float), cudaMemcpyDefault, h->stream));
-    LBMX_CUDA(h, cudaMemcpyAsync(h->staging + n, u, 2 * n * sizeof(float), cudaMemcpyDefault, h->stream));
     if (force) {
         lbmx_status st = upload_force(h, force);
         if (st != LBMX_OK) return st;
     }
+    SpareUse use(*h);
+    if (!h->staging) LBMX_CUDA(h, device_alloc(&h->staging, (size_t)3 * n * sizeof(float)));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->staging, rho, n * sizeof(float), cudaMemcpyDefault, h->stream));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->staging + n, u, 2 * n * sizeof(float), cudaMemcpyDefault, h->stream));
     StepArgs a = base_args(h);
     a.rho_out = h->rho_out;
     a.u_out = h->u_out;
@@ -1002,6 +1052,7 @@ static lbmx_status run_pair(lbmx_handle* h, bool store, bool check, bool sums, b
     }
     // the state is in the other buffers now
     std::swap(h->f, h->f2);
+    std::swap(h->f_alloc, h->f2_alloc);
     std::swap(h->edge, h->edge2);
     std::swap(h->tmap, h->tmap2);
     std::swap(h->pair_tmap[0], h->pair_tmap[1]);
@@ -1032,7 +1083,7 @@ static bool capturing(lbmx_handle* h) {
 // pairs; with the kinetic energy 160 and 183; without sums 111 and 108).
 static bool can_pair(lbmx_handle* h, bool every_step_sums) {
     if (capturing(h) || h->captured) return false;
-    if (!(h->pair_ready || h->pair_stale) || h->batches->load() > 0 || h->nm > 0) return false;
+    if (!h->f2 || !(h->pair_ready || h->pair_stale) || h->batches->load() > 0 || h->nm > 0) return false;
     if (every_step_sums && h->pair_shape == 0 && elem_size(h->p.storage) == 2) return false;
     return !h->pair_stale || (rebuild_special(h) == LBMX_OK && h->pair_ready);
 }
@@ -1051,6 +1102,7 @@ lbmx_status lbmx_step_ex(lbmx_handle* h, int32_t nsteps, uint32_t flags) {
     if (!h->initialized) return fail(h, LBMX_ERR_NOT_INITIALIZED, "lbmx_step: call lbmx_init_from_fields first");
     if (nsteps < 0) return fail(h, LBMX_ERR_INVALID_ARGUMENT, "lbmx_step: nsteps < 0");
     cudaSetDevice(h->p.device);
+    SpareUse use(*h);
     const bool check = (flags & LBMX_STEP_CHECK_FINITE) != 0;
     if (check) LBMX_CUDA(h, cudaMemsetAsync(h->error_word, 0, sizeof(unsigned int), h->stream));
     const bool ke = (flags & LBMX_STEP_KINETIC_ENERGY) != 0;
@@ -1079,6 +1131,7 @@ lbmx_status lbmx_step_sums(lbmx_handle* h, int32_t nsteps, uint32_t flags, doubl
     if (!h->initialized) return fail(h, LBMX_ERR_NOT_INITIALIZED, "lbmx_step_sums: call lbmx_init_from_fields first");
     if (nsteps < 0) return fail(h, LBMX_ERR_INVALID_ARGUMENT, "lbmx_step_sums: nsteps < 0");
     cudaSetDevice(h->p.device);
+    SpareUse use(*h);
     const bool check = (flags & LBMX_STEP_CHECK_FINITE) != 0;
     if (check) LBMX_CUDA(h, cudaMemsetAsync(h->error_word, 0, sizeof(unsigned int), h->stream));
     // device memory and pinned host memory: the step kernel writes each
@@ -1237,7 +1290,7 @@ lbmx_status lbmx_get_populations(lbmx_handle* h, float* out) {
     if (!h->initialized) return fail(h, LBMX_ERR_NOT_INITIALIZED, "lbmx_get_populations: not initialized");
     cudaSetDevice(h->p.device);
     const long long n = (long long)h->g.nx * h->g.ny;
-    if (!h->pop_out) LBMX_CUDA(h, cudaMalloc((void**)&h->pop_out, (size_t)9 * n * sizeof(float)));
+    if (!h->pop_out) LBMX_CUDA(h, device_alloc(&h->pop_out, (size_t)9 * n * sizeof(float)));
     StepArgs a = base_args(h);
     // parity and rest plane of the last step taken (init looks like a parity-0 step)
     set_step(h, a, h->t);
@@ -1317,7 +1370,7 @@ lbmx_status lbmx_opt_partials(lbmx_handle* h, int64_t* sums3) {
     if (!h->initialized) return fail(h, LBMX_ERR_NOT_INITIALIZED, "lbmx_opt_partials: not initialized");
     if (h->p.op != LBMX_CM_OPT) return fail(h, LBMX_ERR_UNSUPPORTED, "lbmx_opt_partials: the operator is not CM_OPT");
     cudaSetDevice(h->p.device);
-    if (!h->raw_sums) LBMX_CUDA(h, cudaMalloc((void**)&h->raw_sums, kNumSums * sizeof(long long)));
+    if (!h->raw_sums) LBMX_CUDA(h, device_alloc(&h->raw_sums, kNumSums * sizeof(long long)));
     const long long s = h->t + 1;
     StepArgs a = base_args(h);
     set_step(h, a, s);
@@ -1441,18 +1494,18 @@ lbmx_status lbmx_ibm_set_markers(lbmx_handle* h, const float* xy, int32_t n) {
     h->nm = n;
     h->npatch = np;
     h->stencil = S;
-    LBMX_CUDA(h, cudaMalloc((void**)&h->patch_nodes, np * sizeof(int)));
-    LBMX_CUDA(h, cudaMalloc((void**)&h->sten_idx, (size_t)n * S2 * sizeof(int)));
-    LBMX_CUDA(h, cudaMalloc((void**)&h->sten_w, (size_t)n * S2 * sizeof(float)));
-    LBMX_CUDA(h, cudaMalloc((void**)&h->marker_u, 2 * (size_t)n * sizeof(float)));
-    LBMX_CUDA(h, cudaMalloc((void**)&h->marker_rho, (size_t)n * sizeof(float)));
-    LBMX_CUDA(h, cudaMalloc((void**)&h->marker_force, 2 * (size_t)n * sizeof(float)));
-    LBMX_CUDA(h, cudaMalloc((void**)&h->ibm_force, 2 * (size_t)g.plane * sizeof(float)));
+    LBMX_CUDA(h, device_alloc(&h->patch_nodes, np * sizeof(int)));
+    LBMX_CUDA(h, device_alloc(&h->sten_idx, (size_t)n * S2 * sizeof(int)));
+    LBMX_CUDA(h, device_alloc(&h->sten_w, (size_t)n * S2 * sizeof(float)));
+    LBMX_CUDA(h, device_alloc(&h->marker_u, 2 * (size_t)n * sizeof(float)));
+    LBMX_CUDA(h, device_alloc(&h->marker_rho, (size_t)n * sizeof(float)));
+    LBMX_CUDA(h, device_alloc(&h->marker_force, 2 * (size_t)n * sizeof(float)));
+    LBMX_CUDA(h, device_alloc(&h->ibm_force, 2 * (size_t)g.plane * sizeof(float)));
     LBMX_CUDA(h, cudaMemcpy(h->patch_nodes, nodes.data(), np * sizeof(int), cudaMemcpyHostToDevice));
     LBMX_CUDA(h, cudaMemcpy(h->sten_idx, sidx.data(), sidx.size() * sizeof(int), cudaMemcpyHostToDevice));
     LBMX_CUDA(h, cudaMemcpy(h->sten_w, sw.data(), sw.size() * sizeof(float), cudaMemcpyHostToDevice));
     const std::vector<int> spread = lbmx::ibm_build_spread(np, sidx);
-    LBMX_CUDA(h, cudaMalloc((void**)&h->spread, spread.size() * sizeof(int)));
+    LBMX_CUDA(h, device_alloc(&h->spread, spread.size() * sizeof(int)));
     LBMX_CUDA(h, cudaMemcpy(h->spread, spread.data(), spread.size() * sizeof(int), cudaMemcpyHostToDevice));
     LBMX_CUDA(h, cudaMemset(h->ibm_force, 0, 2 * (size_t)g.plane * sizeof(float)));
     LBMX_CUDA(h, cudaMemset(h->marker_force, 0, 2 * (size_t)n * sizeof(float)));

@@ -119,7 +119,7 @@ static lbmx_status refresh(lbmx_batch* b) {
         b->host_args.size() == args.size() && memcmp(b->host_args.data(), args.data(), args.size() * sizeof(StepArgs)) == 0;
     if (same_args && b->args_tile_w == tw && b->args_tile_h == th) return LBMX_OK;
     drop_graphs(b);
-    if (!b->d_args) BATCH_CUDA(b, cudaMalloc((void**)&b->d_args, args.size() * sizeof(StepArgs)));
+    if (!b->d_args) BATCH_CUDA(b, device_alloc(&b->d_args, args.size() * sizeof(StepArgs)));
     BATCH_CUDA(b, cudaMemcpyAsync(b->d_args, args.data(), args.size() * sizeof(StepArgs), cudaMemcpyHostToDevice,
                                   b->stream));
     // TMA descriptors and, per parity, the work list
@@ -127,7 +127,7 @@ static lbmx_status refresh(lbmx_batch* b) {
     for (int l = 0; l < n; l++)
         if (!encode_population_map(b->lat[l], &maps[l], tw, th))
             return bfail(b, LBMX_ERR_CUDA, "lbmx_batch: cannot build the TMA descriptor of lattice %d", l);
-    if (!b->d_tmaps) BATCH_CUDA(b, cudaMalloc((void**)&b->d_tmaps, (size_t)n * sizeof(CUtensorMap)));
+    if (!b->d_tmaps) BATCH_CUDA(b, device_alloc(&b->d_tmaps, (size_t)n * sizeof(CUtensorMap)));
     BATCH_CUDA(b, cudaMemcpyAsync(b->d_tmaps, maps.data(), (size_t)n * sizeof(CUtensorMap), cudaMemcpyHostToDevice,
                                   b->stream));
     // Per parity, each lattice's tiles, then its special chunks: a chunk is
@@ -149,7 +149,7 @@ static lbmx_status refresh(lbmx_batch* b) {
         if ((int)items[p].size() > b->items_cap[p]) {
             cudaFree(b->d_items[p]);
             b->d_items[p] = nullptr;
-            BATCH_CUDA(b, cudaMalloc((void**)&b->d_items[p], items[p].size() * sizeof(int2)));
+            BATCH_CUDA(b, device_alloc(&b->d_items[p], items[p].size() * sizeof(int2)));
             b->items_cap[p] = (int)items[p].size();
         }
         BATCH_CUDA(b, cudaMemcpyAsync(b->d_items[p], items[p].data(), items[p].size() * sizeof(int2),
@@ -367,10 +367,10 @@ lbmx_status lbmx_batch_create(lbmx_handle* const* lattices, int32_t count, lbmx_
             b->stream_events.push_back(e);
         }
     }
-    if (cudaMalloc((void**)&b->counter, sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc((void**)&b->done, sizeof(unsigned int)) != cudaSuccess ||
-        cudaMalloc((void**)&b->error_word, sizeof(unsigned int)) != cudaSuccess ||
-        cudaMalloc((void**)&b->step, sizeof(unsigned int)) != cudaSuccess)
+    if (device_alloc(&b->counter, sizeof(unsigned long long)) != cudaSuccess ||
+        device_alloc(&b->done, sizeof(unsigned int)) != cudaSuccess ||
+        device_alloc(&b->error_word, sizeof(unsigned int)) != cudaSuccess ||
+        device_alloc(&b->step, sizeof(unsigned int)) != cudaSuccess)
         return cleanup(LBMX_ERR_OUT_OF_MEMORY, "cudaMalloc failed");
     cudaMemsetAsync(b->step, 0, sizeof(unsigned int), b->stream);
     cudaMemsetAsync(b->counter, 0, sizeof(unsigned long long), b->stream);
@@ -461,7 +461,7 @@ lbmx_status lbmx_batch_autotune(lbmx_batch* b, int32_t trial_steps, lbmx_batch_c
         total += (fb[l] + eb[l] + 255) / 256 * 256;
     }
     char* snap = nullptr;
-    BATCH_CUDA(b, cudaMalloc((void**)&snap, total));
+    BATCH_CUDA(b, device_alloc(&snap, total));
     if ((st = wait_lattices(b)) != LBMX_OK) {
         cudaFree(snap);
         return st;

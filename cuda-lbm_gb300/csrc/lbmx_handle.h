@@ -11,7 +11,8 @@
 #include "lbmx.h"
 #include "lbmx_internal.h"
 
-struct lbmx_handle {
+struct lbmx_handle : lbmx::Spare {
+    bool give_back() override;
     lbmx_params p;
     lbmx::Geometry g;
     cudaStream_t stream = nullptr;
@@ -71,7 +72,8 @@ struct lbmx_handle {
     int* tile_order = nullptr;          // tiles away from the IBM patch, then the others (null without markers)
     int dep_tile = 0;                   // tiles away from the patch
     int nspecial = 0, special_chunks = 0, tiles_x = 0, tiles_y = 0, num_ctas = 0, num_sms = 1;
-    void* f_alloc = nullptr;  // population allocation (f and f2) including the guard elements
+    void* f_alloc = nullptr;   // population allocation including the guard elements
+    void* f2_alloc = nullptr;  // the second one's
     float* edge_alloc = nullptr;  // aux, edge and edge2
     double* mail = nullptr;       // pinned host words a readback leaves sums and error word in
     void* words = nullptr;        // partials, sums, counters, averages, error word
@@ -80,7 +82,8 @@ struct lbmx_handle {
     unsigned long long* tile_counter = nullptr;
     // Two-step launches (lbmx_pair_kernels.cuh): the second population buffer
     // and edge store, which a pair writes and then swaps with f and edge;
-    // null where there is no room for them (every step is then a single one)
+    // null where there is no room for them or they were given back (every
+    // step is then a single one); used with the handle's `busy` held
     void* f2 = nullptr;
     float* edge2 = nullptr;
     CUtensorMap tmap2;                // f2's descriptor for the single-step tiles

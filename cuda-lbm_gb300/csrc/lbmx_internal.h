@@ -4,9 +4,40 @@
 #include <cuda.h>  // CUtensorMap (the descriptor type only; no driver calls are linked)
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <thread>
+
 #include "lbmx.h"
 
 namespace lbmx {
+
+// Device memory an object holds beyond what it needs (a lattice's second
+// population buffer, an adjoint's kept segment): given back when an
+// allocation of any of the library's objects finds the device full, so that
+// everything fits that fits without it.
+struct Spare {
+    int device = 0;
+    std::atomic<bool> busy{false};     // held while a call uses it
+    virtual bool give_back() = 0;      // frees it (with `busy` held); false: there was none
+    virtual ~Spare() = default;
+};
+void spare_add(Spare* s);
+void spare_remove(Spare* s);
+// cudaMalloc on the current device, spares given back one by one as needed
+cudaError_t device_alloc(void** p, size_t bytes);
+template <typename T>
+inline cudaError_t device_alloc(T** p, size_t bytes) {
+    return device_alloc(reinterpret_cast<void**>(p), bytes);
+}
+// Holds a spare for the length of a call.  A give-back by another thread in
+// the meantime is waited for.
+struct SpareUse {
+    Spare& s;
+    explicit SpareUse(Spare& spare) : s(spare) {
+        while (s.busy.exchange(true)) std::this_thread::yield();
+    }
+    ~SpareUse() { s.busy = false; }
+};
 
 // Geometry and storage of one lattice in HBM.
 //

@@ -412,9 +412,9 @@ lbmx_status lbmx_tangent_create(const lbmx_params* p, const uint8_t* flags, int3
         return LBMX_ERR_OUT_OF_MEMORY;
     };
     const size_t state = (size_t)18 * n * sizeof(float);
-    if (cudaMalloc((void**)&t->flags, (size_t)n) != cudaSuccess || cudaMalloc((void**)&t->buf[0], state) != cudaSuccess ||
-        cudaMalloc((void**)&t->buf[1], state) != cudaSuccess ||
-        cudaMalloc((void**)&t->mom, (size_t)6 * n * sizeof(float)) != cudaSuccess)
+    if (device_alloc(&t->flags, (size_t)n) != cudaSuccess || device_alloc(&t->buf[0], state) != cudaSuccess ||
+        device_alloc(&t->buf[1], state) != cudaSuccess ||
+        device_alloc(&t->mom, (size_t)6 * n * sizeof(float)) != cudaSuccess)
         return bail("cudaMalloc failed");
     if (p->stream) {
         t->stream = (cudaStream_t)p->stream;
@@ -433,7 +433,7 @@ lbmx_status lbmx_tangent_set_state(lbmx_tangent* t, const float* rho, const floa
     if (!t || !rho || !u) return tfail(t, LBMX_ERR_INVALID_ARGUMENT, "lbmx_tangent_set_state: NULL argument");
     cudaSetDevice(t->p.device);
     float* tmp = nullptr;
-    TAN_CUDA(t, cudaMalloc((void**)&tmp, (size_t)3 * t->n * sizeof(float)));
+    TAN_CUDA(t, device_alloc(&tmp, (size_t)3 * t->n * sizeof(float)));
     cudaMemcpyAsync(tmp, rho, (size_t)t->n * sizeof(float), cudaMemcpyDefault, t->stream);
     cudaMemcpyAsync(tmp + t->n, u, (size_t)2 * t->n * sizeof(float), cudaMemcpyDefault, t->stream);
     tan_init_kernel<<<node_grid(t), dim3(kTanBX, kTanBY), 0, t->stream>>>(t->args, tmp, tmp + t->n, t->buf[0],
@@ -474,18 +474,18 @@ lbmx_status lbmx_tangent_set_markers(lbmx_tangent* t, const float* xy, int32_t n
     t->nm = n;
     t->npatch = np;
     t->stencil = two ? 2 : 4;
-    TAN_CUDA(t, cudaMalloc((void**)&t->patch_nodes, np * sizeof(int)));
-    TAN_CUDA(t, cudaMalloc((void**)&t->sten_idx, sidx.size() * sizeof(int)));
-    TAN_CUDA(t, cudaMalloc((void**)&t->sten_w, sw.size() * sizeof(float)));
-    TAN_CUDA(t, cudaMalloc((void**)&t->marker_u, 2 * (size_t)n * sizeof(D)));
-    TAN_CUDA(t, cudaMalloc((void**)&t->marker_rho, (size_t)n * sizeof(D)));
-    TAN_CUDA(t, cudaMalloc((void**)&t->marker_force, 2 * (size_t)n * sizeof(D)));
-    TAN_CUDA(t, cudaMalloc((void**)&t->ibm_force, 2 * (size_t)t->n * sizeof(D)));
+    TAN_CUDA(t, device_alloc(&t->patch_nodes, np * sizeof(int)));
+    TAN_CUDA(t, device_alloc(&t->sten_idx, sidx.size() * sizeof(int)));
+    TAN_CUDA(t, device_alloc(&t->sten_w, sw.size() * sizeof(float)));
+    TAN_CUDA(t, device_alloc(&t->marker_u, 2 * (size_t)n * sizeof(D)));
+    TAN_CUDA(t, device_alloc(&t->marker_rho, (size_t)n * sizeof(D)));
+    TAN_CUDA(t, device_alloc(&t->marker_force, 2 * (size_t)n * sizeof(D)));
+    TAN_CUDA(t, device_alloc(&t->ibm_force, 2 * (size_t)t->n * sizeof(D)));
     TAN_CUDA(t, cudaMemcpy(t->patch_nodes, nodes.data(), np * sizeof(int), cudaMemcpyHostToDevice));
     TAN_CUDA(t, cudaMemcpy(t->sten_idx, sidx.data(), sidx.size() * sizeof(int), cudaMemcpyHostToDevice));
     TAN_CUDA(t, cudaMemcpy(t->sten_w, sw.data(), sw.size() * sizeof(float), cudaMemcpyHostToDevice));
     const std::vector<int> spread = ibm_build_spread(np, sidx);
-    TAN_CUDA(t, cudaMalloc((void**)&t->spread, spread.size() * sizeof(int)));
+    TAN_CUDA(t, device_alloc(&t->spread, spread.size() * sizeof(int)));
     TAN_CUDA(t, cudaMemcpy(t->spread, spread.data(), spread.size() * sizeof(int), cudaMemcpyHostToDevice));
     TAN_CUDA(t, cudaMemset(t->ibm_force, 0, 2 * (size_t)t->n * sizeof(D)));
     TAN_CUDA(t, cudaMemset(t->marker_force, 0, 2 * (size_t)n * sizeof(D)));
@@ -513,7 +513,7 @@ lbmx_status lbmx_tangent_run(lbmx_tangent* t, int32_t nsteps, double* series) {
     if (series && nsteps > t->series_cap) {
         cudaFree(t->series);
         t->series = nullptr;
-        TAN_CUDA(t, cudaMalloc((void**)&t->series, (size_t)4 * nsteps * sizeof(double)));
+        TAN_CUDA(t, device_alloc(&t->series, (size_t)4 * nsteps * sizeof(double)));
         t->series_cap = nsteps;
     }
     if (series) TAN_CUDA(t, cudaMemsetAsync(t->series, 0, (size_t)4 * nsteps * sizeof(double), t->stream));

@@ -26,6 +26,7 @@ QUIRK_REST_LAG, QUIRK_ZOUHE_LEFT, QUIRK_MRT_FORCE, QUIRK_IBM_2X2, QUIRK_IBM_CLAM
 QUIRKS_REFERENCE = 0x1F
 OPTION_LAGGED_AVERAGES = 1
 OPTION_ROUND_NEAREST = 2
+OPTION_SINGLE_BUFFER = 4
 STEP_STORE_MOMENTS, STEP_CHECK_FINITE, STEP_SUMS, STEP_KINETIC_ENERGY = 1, 2, 4, 8
 
 STATUS = {0: "OK", 1: "INVALID_ARGUMENT", 2: "OUT_OF_MEMORY", 3: "CUDA", 4: "INVALID_FLAGS",

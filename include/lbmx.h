@@ -86,7 +86,9 @@ enum {
 /* lbmx_params.options */
 enum {
     LBMX_OPTION_LAGGED_AVERAGES = 1u << 0, /* CM_OPT: use the previous step's grid averages (one pass) */
-    LBMX_OPTION_ROUND_NEAREST = 1u << 1    /* 16-bit storage rounds to nearest instead of stochastically */
+    LBMX_OPTION_ROUND_NEAREST = 1u << 1,   /* 16-bit storage rounds to nearest instead of stochastically */
+    LBMX_OPTION_SINGLE_BUFFER = 1u << 2    /* no second population buffer (lbmx_create) and no states kept for a
+                                            * backward run (lbmx_adjoint_forward): the smallest footprint */
 };
 
 /* lbmx_step_ex flags */
@@ -129,7 +131,10 @@ void lbmx_params_default(lbmx_params* p);
 
 /* Replaces LBM<2>::allocate<S>() + send_consts<S>() (src/core/lbm.cuh:92-125, :63-82).
  * Allocates a second population buffer, for two steps per launch, while the
- * device keeps at least half of its memory free beside it. */
+ * device keeps at least half of its memory free beside it (never with
+ * LBMX_OPTION_SINGLE_BUFFER).  It is freed when a later allocation of this
+ * library finds the device full; the lattice then steps one step a launch,
+ * with the same results. */
 lbmx_status lbmx_create(const lbmx_params* p, lbmx_handle** out);
 
 /* Replaces ~LBM() / LBM::free() (src/core/lbm.cuh:127-140, :379-381). */
@@ -345,7 +350,8 @@ lbmx_status lbmx_moment_sums_noalloc(const float* rho, const float* u, int64_t n
  * exactly, and the populations are recomputed from checkpoints taken every
  * `checkpoint_every` steps, so memory is (steps / every + every) states
  * (the segment's `every` already in the forward run where the device has
- * them to spare).
+ * them to spare and LBMX_OPTION_SINGLE_BUFFER is not set; freed, like a
+ * lattice's second buffer, when another allocation needs the memory).
  * FP32 populations; any operator; fluid, bounce-back (where it reads no
  * population from outside the domain) and half-way / moving walls; no IBM. */
 typedef struct lbmx_adjoint lbmx_adjoint;

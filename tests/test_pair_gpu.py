@@ -300,3 +300,100 @@ def test_a_lattice_that_left_its_batch_is_as_fast_as_before():
         best.append(min(times))
         L.close()
     assert best[1] < 1.4 * best[0], best
+
+
+def test_spare_buffers_make_way_for_a_new_lattice():
+    """On a full device the second buffer of one lattice is given back for
+    the allocations of another, which fit without it; the first goes on."""
+    import torch
+    import lbmx
+    n = 4096  # 0.6 GB a buffer; given back: that less 0.2 GB of staging
+
+    def start():
+        L = lbmx.Lattice(n, n, op=lbmx.MRT, omega=1.3, periodic=(True, True))
+        L.init(rho, u)
+        return L
+
+    r = np.random.default_rng(4)
+    rho = (1 + 0.01 * r.standard_normal((n, n))).astype(np.float32)
+    u = (0.01 * r.standard_normal((2, n, n))).astype(np.float32)
+    B = start()
+    for _ in range(2 + 3 + 2):
+        B.step(1)
+    want = B.moments()
+    B.close()
+    torch.cuda.empty_cache()
+    A = start()
+    A.step(2)
+    A.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    full = torch.empty(free - (128 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        C2 = lbmx.Lattice(2048, 2048, op=lbmx.MRT, omega=1.3, periodic=(True, True))  # 0.25 GB
+    finally:
+        del full
+        torch.cuda.empty_cache()
+    C2.close()
+    A.step(3)
+    A.step(2)
+    for x, y in zip(A.moments(), want):
+        np.testing.assert_array_equal(x, y)
+    # and its init fields have their own staging now
+    A.init(rho, u)
+    A.step(7)
+    for x, y in zip(A.moments(), want):
+        np.testing.assert_array_equal(x, y)
+
+
+def test_single_buffer_option():
+    import torch
+    import lbmx
+    n = 2048
+    used = []
+    torch.cuda.synchronize()
+    for options in (0, lbmx.OPTION_SINGLE_BUFFER):
+        before = torch.cuda.mem_get_info()[0]
+        L = lbmx.Lattice(n, n, op=lbmx.BGK, omega=1.3, periodic=(True, True), options=options)
+        used.append(before - torch.cuda.mem_get_info()[0])
+        L.close()
+    # 36 bytes a node of second buffer against 12 of staging
+    assert used[0] - used[1] > 20 * n * n, used
+    c = C.random_state(C.cavity_moving_wall(70, 37, op=C.BGK), seed=5)
+    A, B = C.make_lattice(c), C.make_lattice(c, options=lbmx.OPTION_SINGLE_BUFFER)
+    for n in (2, 3, 4):
+        A.step(n)
+        B.step(n)
+        same(A, B)
+
+
+def test_adjoint_segment_makes_way():
+    """The segment kept by a forward run is given back to another object's
+    allocation and recomputed by the backward run, to the same gradient."""
+    import torch
+    import lbmx
+    nx = ny = 1024  # 36 MB a state, 15 of them in the segment
+    r = np.random.default_rng(7)
+    rho, u = np.ones((ny, nx), np.float32), (0.01 * r.standard_normal((2, ny, nx))).astype(np.float32)
+    gamma = (0.1 * r.random((ny, nx))).astype(np.float32)
+    w = np.zeros((3, ny, nx), np.float32)
+    w[1] = r.random((ny, nx))
+    a = lbmx.Adjoint(nx, ny, op=lbmx.CM, omega=1.2, periodic=(True, True), checkpoint_every=16)
+    a.set_state(rho, u)
+    a.set_gamma(gamma)
+    a.set_objective(w, 1)
+    a.forward(20)
+    want, scalars = a.backward()
+    a.forward(16)
+    a.forward(20)
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    full = torch.empty(free - (128 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        L = lbmx.Lattice(2048, 2048, op=lbmx.MRT, omega=1.3, periodic=(True, True))
+    finally:
+        del full
+        torch.cuda.empty_cache()
+    L.close()
+    got, s = a.backward()
+    np.testing.assert_array_equal(got, want)
+    assert s == scalars
