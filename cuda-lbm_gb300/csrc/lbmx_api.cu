@@ -481,9 +481,11 @@ __global__ void __launch_bounds__(32 * kReadbackRows) readback_kernel(const Read
     }
 }
 
-// Device memory the handle's kernels may write (null: nothing to write).
+// Device memory the handle's kernels may write floats to (null: nothing to
+// write); a field that does not start on four bytes is copied.
 static bool device_writable(const lbmx_handle* h, const void* p) {
     if (!p) return true;
+    if (reinterpret_cast<uintptr_t>(p) % sizeof(float) != 0) return false;
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();

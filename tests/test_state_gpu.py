@@ -4,6 +4,7 @@ A checkpoint holds the dynamic state only (populations in storage form, the
 edge store, the step count, the CM_OPT averages) plus a CRC-32; a handle
 built with the same params, flags, force and markers continues bit for bit.
 """
+import ctypes
 import os
 
 import numpy as np
@@ -250,3 +251,24 @@ def test_kinetic_energy_decays_at_the_taylor_green_rate():
     # 1.4e-8 per node per step, 8e-6 of the mass in 600 steps, as much as a
     # plain float32 numpy BGK step drifts on this case (float64: 1e-16)
     assert np.all(np.abs(s[:, 0] - 64 * 64) <= 5e-5 * 64 * 64)
+
+
+@pytest.mark.parametrize("nx", [64, 67])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 4, 8, 16])
+def test_moments_into_device_fields_at_any_address(nx, offset):
+    """Fields in device memory at every alignment, odd ones by copies."""
+    import torch
+    ny = 19
+    L = C.make_lattice(C.random_state(C.cavity_moving_wall(nx, ny, op=C.BGK), seed=3))
+    L.step(3)
+    rho, u, sums = L.moments()
+    n = nx * ny
+    buf = torch.zeros(12 * n + 64, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    base = buf.data_ptr() + offset
+    s = (ctypes.c_double * 3)()
+    L._check(L.lib.lbmx_moments(L.h, base, base + 4 * n, s))
+    got = np.frombuffer(buf.cpu().numpy().tobytes()[offset:offset + 12 * n], np.float32)
+    np.testing.assert_array_equal(got[:n].reshape(ny, nx), rho)
+    np.testing.assert_array_equal(got[n:].reshape(2, ny, nx), u)
+    assert list(s) == list(sums)
