@@ -1490,7 +1490,7 @@ lbmx_status lbmx_ibm_set_markers(lbmx_handle* h, const float* xy, int32_t n) {
     const int bad = lbmx::ibm_build_stencil(g.nx, g.ny, g.pitch, two, hxy.data(), n, sidx, sw, nodes);
     if (bad >= 0) return fail(h, LBMX_ERR_INVALID_ARGUMENT, "lbmx_ibm_set_markers: marker %d is not finite", bad);
     const int np = (int)nodes.size();
-    if (lbmx::ibm_smem_bytes(np, n, S) > 200 * 1024)
+    if (lbmx::ibm_smem_bytes(np, n, S) > kIbmSmemLimit)
         return fail(h, LBMX_ERR_TOO_LARGE, "lbmx_ibm_set_markers: %d markers touch %d nodes; limit is 200 KB of patch state",
                     n, np);
     h->nm = n;

@@ -358,6 +358,9 @@ inline int pair_shape(int nx, int ny, int elem_bytes, int op, int num_sms) {
     }
     return tiles(2) >= num_sms ? 2 : 3;
 }
+// dynamic shared memory an IBM patch may take (the kernels' static arrays fit
+// beside it in the 227 KB of a CTA)
+constexpr int kIbmSmemLimit = 200 * 1024;
 constexpr int kSpecialChunk = kConsumerWarps * 32;  // special nodes per work item (one per consumer thread)
 // guard elements before and after the population planes: staged row copies
 // reach one 16-byte chunk beyond a row segment on each side

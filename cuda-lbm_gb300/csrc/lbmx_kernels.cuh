@@ -1188,14 +1188,15 @@ template <typename T>
 cudaError_t launch_ibm_step(const StepArgs& a, const IbmArgs& ib, cudaStream_t s) {
     if (ib.npatch <= 0) return cudaSuccess;
     const size_t smem = ibm_fast_smem_bytes(ib.npatch, ib.nm, ib.stencil);
-    // the attribute grows with the patch: raise it when a larger one comes
-    static int configured[64] = {0};
+    // the same limit for every patch, set once per device: handles in several
+    // threads share it
+    static unsigned long long configured = 0;
     int dev = 0;
     cudaGetDevice(&dev);
-    if ((int)smem > configured[dev & 63]) {
-        cudaError_t e = cudaFuncSetAttribute(ibm_step_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (!(configured >> (dev & 63) & 1ull)) {
+        cudaError_t e = cudaFuncSetAttribute(ibm_step_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kIbmSmemLimit);
         if (e != cudaSuccess) return e;
-        configured[dev & 63] = (int)smem;
+        configured |= 1ull << (dev & 63);
     }
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));

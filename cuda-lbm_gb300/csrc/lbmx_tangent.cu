@@ -468,7 +468,7 @@ lbmx_status lbmx_tangent_set_markers(lbmx_tangent* t, const float* xy, int32_t n
     const int bad = ibm_build_stencil(t->p.nx, t->p.ny, t->p.nx, two, hxy.data(), n, sidx, sw, nodes);
     if (bad >= 0) return tfail(t, LBMX_ERR_INVALID_ARGUMENT, "lbmx_tangent_set_markers: marker %d is not finite", bad);
     const int np = (int)nodes.size();
-    if (ibm_smem_bytes_of<D>(np, n, two ? 2 : 4) > 200 * 1024)
+    if (ibm_smem_bytes_of<D>(np, n, two ? 2 : 4) > kIbmSmemLimit)
         return tfail(t, LBMX_ERR_TOO_LARGE,
                      "lbmx_tangent_set_markers: %d markers touch %d nodes; limit is 200 KB of patch state", n, np);
     t->nm = n;
@@ -492,14 +492,8 @@ lbmx_status lbmx_tangent_set_markers(lbmx_tangent* t, const float* xy, int32_t n
     std::vector<uint8_t> marked = t->flags_host;
     for (int node : nodes) marked[(size_t)node] |= kPatchBit;
     TAN_CUDA(t, cudaMemcpy(t->flags, marked.data(), marked.size(), cudaMemcpyHostToDevice));
-    // the kernel's limit only grows: tangents with smaller patches share it
-    static int configured[64] = {0};
-    const int smem = (int)ibm_smem_bytes_of<D>(np, n, t->stencil);
-    int& limit = configured[t->p.device & 63];
-    if (smem > limit) {
-        TAN_CUDA(t, cudaFuncSetAttribute(tan_ibm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        limit = smem;
-    }
+    // always the same limit: tangents of any patch, in any threads, share it
+    TAN_CUDA(t, cudaFuncSetAttribute(tan_ibm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIbmSmemLimit));
     t->args.ibm_force = t->ibm_force;
     t->args.forced = 1;
     return LBMX_OK;

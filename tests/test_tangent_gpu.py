@@ -7,6 +7,9 @@ the cavity's velocity field (lid velocity) and of a forced channel's velocity
 (body force) must match central finite differences of the FP64 oracle to
 1e-3 relative.
 """
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -167,3 +170,42 @@ def test_markers_off_walls_and_across_blocks(op):
         scale = np.abs(want).max()
         assert np.abs(got[:, :2] - want).max() <= 1e-4 * scale
         assert np.isfinite(other.run(3)).all()
+
+
+THREADS = """
+import sys, threading
+sys.path[:0] = %r
+import numpy as np
+import cases as C, lbmx
+sizes = [12, 300, 40, 200, 24, 100]
+start = threading.Barrier(len(sizes))
+out = [None] * len(sizes)
+
+def run(i):
+    mk = C.cylinder_markers(60.3, 41.7, 1.0 + sizes[i] / 12.0, sizes[i])
+    c = C.channel(128, 84, op=C.BGK, nu=0.04, u_in=0.05, inlet="parabolic", outlet="zouhe_p", markers=mk)
+    t = lbmx.Tangent(c["nx"], c["ny"], lbmx.TANGENT_U_BC, op=c["op"], omega=c["omega"], S=c["S"],
+                     periodic=c["periodic"], flags=c["flags"], u_bc=c["u_bc"], rho_out=c["rho_out"])
+    t.set_state(np.asarray(c["rho"], np.float32), np.asarray(c["u"], np.float32))
+    L = C.make_lattice(dict(c, markers=None))
+    start.wait()
+    t.set_markers(mk)
+    L.set_markers(mk)
+    L.step(1)
+    start.wait()
+    out[i] = np.isfinite(t.run(3)).all()
+    L.step(2)
+    L.synchronize()
+
+ts = [threading.Thread(target=run, args=(i,)) for i in range(len(sizes))]
+[t.start() for t in ts]
+[t.join() for t in ts]
+assert all(out), out
+"""
+
+
+def test_patches_of_several_threads_share_the_kernels():
+    """Small and large patches set at the same moment in a fresh process: no
+    thread lowers the shared-memory limit that another one's kernel needs."""
+    r = subprocess.run([sys.executable, "-c", THREADS % (sys.path,)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
