@@ -1232,7 +1232,9 @@ lbmx_status lbmx_adjoint_create(const lbmx_params* p, const uint8_t* flags, int3
         if (cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking) != cudaSuccess) return bail("no stream");
         a->own_stream = true;
     }
-    cudaMemcpy(a->flags, fl.data(), fl.size(), cudaMemcpyHostToDevice);
+    if (cudaMemcpyAsync(a->flags, fl.data(), fl.size(), cudaMemcpyHostToDevice, a->stream) != cudaSuccess ||
+        cudaStreamSynchronize(a->stream) != cudaSuccess)
+        return bail("flag upload");
     a->args.flags = a->flags;
     a->device = p->device;
     spare_add(a);

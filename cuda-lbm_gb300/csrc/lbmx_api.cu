@@ -159,8 +159,11 @@ StepArgs lbmx::base_args(const lbmx_handle* h) {
 }
 
 // A device list in a buffer that only grows (a cudaFree / cudaMalloc pair per
-// list costs about as much as building it).
-static cudaError_t upload_list(const void* src, size_t bytes, void** buf, size_t* cap) {
+// list costs about as much as building it), uploaded on the handle's stream:
+// a blocking copy of pageable memory goes through the legacy stream, may
+// return before the bytes have landed, and a non-blocking stream's kernels do
+// not wait for it.  The caller waits for the stream before src goes.
+static cudaError_t upload_list(lbmx_handle* h, const void* src, size_t bytes, void** buf, size_t* cap) {
     if (!*buf || *cap < bytes) {
         cudaFree(*buf);
         *buf = nullptr;
@@ -169,7 +172,7 @@ static cudaError_t upload_list(const void* src, size_t bytes, void** buf, size_t
         if (e != cudaSuccess) return e;
         *cap = std::max<size_t>(bytes, 4);
     }
-    return bytes ? cudaMemcpy(*buf, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
+    return bytes ? cudaMemcpyAsync(*buf, src, bytes, cudaMemcpyHostToDevice, h->stream) : cudaSuccess;
 }
 
 // General-path nodes of every two-step tile, from the unit lists of the two
@@ -244,10 +247,11 @@ static lbmx_status rebuild_pair_lists(lbmx_handle* h, const std::vector<int>& un
         sp += found[step].size();
     }
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (upload_list(all.data(), all.size() * sizeof(int), (void**)&h->pair_lists, &h->cap_pair_lists) != cudaSuccess) {
+    if (upload_list(h, all.data(), all.size() * sizeof(int), (void**)&h->pair_lists, &h->cap_pair_lists) != cudaSuccess) {
         cudaGetLastError();  // no room for them: single steps
         return LBMX_OK;
     }
+    LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
     h->pair_tiles = nt;
     h->pair_tiles_x = tx;
     h->pair_sp1 = (int)n1;
@@ -374,15 +378,15 @@ static lbmx_status rebuild_special(lbmx_handle* h, bool pair_lists = true) {
     const int indep = by_patch(units), indep0 = by_patch(units0);
     // device copies; null unit bits: none marked
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
-    LBMX_CUDA(h, upload_list(units.data(), units.size() * sizeof(int), (void**)&h->special_units, &h->cap_units));
-    LBMX_CUDA(h, upload_list(units0.data(), units0.size() * sizeof(int), (void**)&h->special_units0, &h->cap_units0));
+    LBMX_CUDA(h, upload_list(h, units.data(), units.size() * sizeof(int), (void**)&h->special_units, &h->cap_units));
+    LBMX_CUDA(h, upload_list(h, units0.data(), units0.size() * sizeof(int), (void**)&h->special_units0, &h->cap_units0));
     h->special_bits = h->special_bits0 = nullptr;
     if (any_interior) {
-        LBMX_CUDA(h, upload_list(bits.data(), bits.size() * sizeof(uint32_t), (void**)&h->bits_buf, &h->cap_bits));
+        LBMX_CUDA(h, upload_list(h, bits.data(), bits.size() * sizeof(uint32_t), (void**)&h->bits_buf, &h->cap_bits));
         h->special_bits = h->bits_buf;
     }
     if (!units0.empty() || h->ghost_mask) {
-        LBMX_CUDA(h, upload_list(bits0.data(), bits0.size() * sizeof(uint32_t), (void**)&h->bits0_buf, &h->cap_bits0));
+        LBMX_CUDA(h, upload_list(h, bits0.data(), bits0.size() * sizeof(uint32_t), (void**)&h->bits0_buf, &h->cap_bits0));
         h->special_bits0 = h->bits0_buf;
     }
     h->nspecial = (int)units.size();
@@ -415,7 +419,9 @@ static lbmx_status rebuild_special(lbmx_handle* h, bool pair_lists = true) {
         h->dep_tile = (int)first.size();
         first.insert(first.end(), last.begin(), last.end());
         LBMX_CUDA(h, device_alloc(&h->tile_order, first.size() * sizeof(int)));
-        LBMX_CUDA(h, cudaMemcpy(h->tile_order, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
+        LBMX_CUDA(h, cudaMemcpyAsync(h->tile_order, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice,
+                                     h->stream));
+        LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
     }
     // Persistent CTAs walk the work list, kCtasPerSm per SM, except in the
     // steps with general-path chunks of a lattice so small that three CTAs
@@ -441,6 +447,7 @@ static lbmx_status rebuild_special(lbmx_handle* h, bool pair_lists = true) {
     };
     split(h->special_chunks, &h->num_ctas, &h->tile_chunk);
     split(h->special_chunks0, &h->num_ctas0, &h->tile_chunk0);
+    LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
     return LBMX_OK;
 }
 
@@ -780,7 +787,7 @@ lbmx_status lbmx_set_flags(lbmx_handle* h, const uint8_t* flags) {
     h->flags_host.assign((size_t)g.plane, 0);
     for (int y = 0; y < g.ny; y++)
         memcpy(&h->flags_host[(size_t)y * g.pitch], &hf[(size_t)y * g.nx], g.nx);
-    LBMX_CUDA(h, cudaMemcpy(h->flags, h->flags_host.data(), (size_t)g.plane, cudaMemcpyHostToDevice));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->flags, h->flags_host.data(), (size_t)g.plane, cudaMemcpyHostToDevice, h->stream));
     h->has_aux_bc = aux;
     h->has_regularized = reg;
     return rebuild_special(h);
@@ -1503,16 +1510,16 @@ lbmx_status lbmx_ibm_set_markers(lbmx_handle* h, const float* xy, int32_t n) {
     LBMX_CUDA(h, device_alloc(&h->marker_rho, (size_t)n * sizeof(float)));
     LBMX_CUDA(h, device_alloc(&h->marker_force, 2 * (size_t)n * sizeof(float)));
     LBMX_CUDA(h, device_alloc(&h->ibm_force, 2 * (size_t)g.plane * sizeof(float)));
-    LBMX_CUDA(h, cudaMemcpy(h->patch_nodes, nodes.data(), np * sizeof(int), cudaMemcpyHostToDevice));
-    LBMX_CUDA(h, cudaMemcpy(h->sten_idx, sidx.data(), sidx.size() * sizeof(int), cudaMemcpyHostToDevice));
-    LBMX_CUDA(h, cudaMemcpy(h->sten_w, sw.data(), sw.size() * sizeof(float), cudaMemcpyHostToDevice));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->patch_nodes, nodes.data(), np * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->sten_idx, sidx.data(), sidx.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->sten_w, sw.data(), sw.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     const std::vector<int> spread = lbmx::ibm_build_spread(np, sidx);
     LBMX_CUDA(h, device_alloc(&h->spread, spread.size() * sizeof(int)));
-    LBMX_CUDA(h, cudaMemcpy(h->spread, spread.data(), spread.size() * sizeof(int), cudaMemcpyHostToDevice));
-    LBMX_CUDA(h, cudaMemset(h->ibm_force, 0, 2 * (size_t)g.plane * sizeof(float)));
-    LBMX_CUDA(h, cudaMemset(h->marker_force, 0, 2 * (size_t)n * sizeof(float)));
-    LBMX_CUDA(h, cudaMemset(h->marker_u, 0, 2 * (size_t)n * sizeof(float)));
-    LBMX_CUDA(h, cudaMemset(h->marker_rho, 0, (size_t)n * sizeof(float)));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->spread, spread.data(), spread.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    LBMX_CUDA(h, cudaMemsetAsync(h->ibm_force, 0, 2 * (size_t)g.plane * sizeof(float), h->stream));
+    LBMX_CUDA(h, cudaMemsetAsync(h->marker_force, 0, 2 * (size_t)n * sizeof(float), h->stream));
+    LBMX_CUDA(h, cudaMemsetAsync(h->marker_u, 0, 2 * (size_t)n * sizeof(float), h->stream));
+    LBMX_CUDA(h, cudaMemsetAsync(h->marker_rho, 0, (size_t)n * sizeof(float), h->stream));
     h->patch_host = nodes;  // patch nodes read the IBM force: general path
     return rebuild_special(h);
 }
@@ -1639,9 +1646,9 @@ lbmx_status lbmx_checkpoint_load(lbmx_handle* h, const char* path) {
     crc = crc32_update(crc, avg, sizeof(avg));
     if (crc != crc_file) return fail(h, LBMX_ERR_INVALID_ARGUMENT, "lbmx_checkpoint_load: %s fails its CRC-32", path);
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
-    LBMX_CUDA(h, cudaMemcpy(h->f, f.data(), f.size(), cudaMemcpyHostToDevice));
-    LBMX_CUDA(h, cudaMemcpy(h->edge, edge.data(), edge.size(), cudaMemcpyHostToDevice));
-    LBMX_CUDA(h, cudaMemcpy(h->avg, avg, sizeof(avg), cudaMemcpyHostToDevice));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->f, f.data(), f.size(), cudaMemcpyHostToDevice, h->stream));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->edge, edge.data(), edge.size(), cudaMemcpyHostToDevice, h->stream));
+    LBMX_CUDA(h, cudaMemcpyAsync(h->avg, avg, sizeof(avg), cudaMemcpyHostToDevice, h->stream));
     LBMX_CUDA(h, copy_edge(h));
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
     h->t = hd.t;

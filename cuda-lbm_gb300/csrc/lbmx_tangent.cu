@@ -422,7 +422,9 @@ lbmx_status lbmx_tangent_create(const lbmx_params* p, const uint8_t* flags, int3
         if (cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) != cudaSuccess) return bail("no stream");
         t->own_stream = true;
     }
-    if (cudaMemcpy(t->flags, fl.data(), fl.size(), cudaMemcpyHostToDevice) != cudaSuccess) return bail("flag upload");
+    if (cudaMemcpyAsync(t->flags, fl.data(), fl.size(), cudaMemcpyHostToDevice, t->stream) != cudaSuccess ||
+        cudaStreamSynchronize(t->stream) != cudaSuccess)
+        return bail("flag upload");
     a.flags = t->flags;
     t->flags_host.swap(fl);
     *out = t;
@@ -457,7 +459,8 @@ lbmx_status lbmx_tangent_set_markers(lbmx_tangent* t, const float* xy, int32_t n
     TAN_CUDA(t, cudaStreamSynchronize(t->stream));
     free_markers(t);
     if (n == 0) {
-        TAN_CUDA(t, cudaMemcpy(t->flags, t->flags_host.data(), t->flags_host.size(), cudaMemcpyHostToDevice));
+        TAN_CUDA(t, cudaMemcpyAsync(t->flags, t->flags_host.data(), t->flags_host.size(), cudaMemcpyHostToDevice, t->stream));
+        TAN_CUDA(t, cudaStreamSynchronize(t->stream));
         return LBMX_OK;
     }
     std::vector<float> hxy(2 * (size_t)n);
@@ -481,17 +484,18 @@ lbmx_status lbmx_tangent_set_markers(lbmx_tangent* t, const float* xy, int32_t n
     TAN_CUDA(t, device_alloc(&t->marker_rho, (size_t)n * sizeof(D)));
     TAN_CUDA(t, device_alloc(&t->marker_force, 2 * (size_t)n * sizeof(D)));
     TAN_CUDA(t, device_alloc(&t->ibm_force, 2 * (size_t)t->n * sizeof(D)));
-    TAN_CUDA(t, cudaMemcpy(t->patch_nodes, nodes.data(), np * sizeof(int), cudaMemcpyHostToDevice));
-    TAN_CUDA(t, cudaMemcpy(t->sten_idx, sidx.data(), sidx.size() * sizeof(int), cudaMemcpyHostToDevice));
-    TAN_CUDA(t, cudaMemcpy(t->sten_w, sw.data(), sw.size() * sizeof(float), cudaMemcpyHostToDevice));
+    TAN_CUDA(t, cudaMemcpyAsync(t->patch_nodes, nodes.data(), np * sizeof(int), cudaMemcpyHostToDevice, t->stream));
+    TAN_CUDA(t, cudaMemcpyAsync(t->sten_idx, sidx.data(), sidx.size() * sizeof(int), cudaMemcpyHostToDevice, t->stream));
+    TAN_CUDA(t, cudaMemcpyAsync(t->sten_w, sw.data(), sw.size() * sizeof(float), cudaMemcpyHostToDevice, t->stream));
     const std::vector<int> spread = ibm_build_spread(np, sidx);
     TAN_CUDA(t, device_alloc(&t->spread, spread.size() * sizeof(int)));
-    TAN_CUDA(t, cudaMemcpy(t->spread, spread.data(), spread.size() * sizeof(int), cudaMemcpyHostToDevice));
-    TAN_CUDA(t, cudaMemset(t->ibm_force, 0, 2 * (size_t)t->n * sizeof(D)));
-    TAN_CUDA(t, cudaMemset(t->marker_force, 0, 2 * (size_t)n * sizeof(D)));
+    TAN_CUDA(t, cudaMemcpyAsync(t->spread, spread.data(), spread.size() * sizeof(int), cudaMemcpyHostToDevice, t->stream));
+    TAN_CUDA(t, cudaMemsetAsync(t->ibm_force, 0, 2 * (size_t)t->n * sizeof(D), t->stream));
+    TAN_CUDA(t, cudaMemsetAsync(t->marker_force, 0, 2 * (size_t)n * sizeof(D), t->stream));
     std::vector<uint8_t> marked = t->flags_host;
     for (int node : nodes) marked[(size_t)node] |= kPatchBit;
-    TAN_CUDA(t, cudaMemcpy(t->flags, marked.data(), marked.size(), cudaMemcpyHostToDevice));
+    TAN_CUDA(t, cudaMemcpyAsync(t->flags, marked.data(), marked.size(), cudaMemcpyHostToDevice, t->stream));
+    TAN_CUDA(t, cudaStreamSynchronize(t->stream));
     // always the same limit: tangents of any patch, in any threads, share it
     TAN_CUDA(t, cudaFuncSetAttribute(tan_ibm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIbmSmemLimit));
     t->args.ibm_force = t->ibm_force;
