@@ -801,22 +801,30 @@ __device__ __forceinline__ void opt_terms(const StepArgs& a, long long off, cons
     v[5] += fix(sqrtf(pxx * pxx + 2.0f * pxy * pxy + pyy * pyy));
 }
 
-// fix() of a pair's sum known to be near `rest`, an even integer: a 32-bit
-// conversion of the difference (exact for t within a factor of two of rest;
-// any t when rest is 0) while that is below one, fix() itself otherwise.
-__device__ __forceinline__ Acc fix_near(float t, float rest) {
-    const float d = t - rest;
-    if (fabsf(d) < 1.0f) return (Acc)__float2int_rn(__fmul_rn(d, kFixScale)) + (Acc)rest * (1ll << 30);
-    return fix(t);
+// fix() of two nodes' terms, each rounded alone, by 32-bit conversions of
+// their products with 2^30 while both are below one, fix() itself otherwise
+// (NaN included).
+__device__ __forceinline__ Acc fix_two(float2 t) {
+    if (fabsf(t.x) < 1.0f && fabsf(t.y) < 1.0f)
+        return (Acc)(__float2int_rn(__fmul_rn(t.x, kFixScale)) + __float2int_rn(__fmul_rn(t.y, kFixScale)));
+    return fix(t.x) + fix(t.y);
+}
+// The same for two densities, with one conversion: above 1/2 and below 3/2
+// their differences from 1 are multiples of 2^-24, and so is the differences'
+// sum, which is below one: exact, as its product with 2^30 is.
+__device__ __forceinline__ Acc fix_two_densities(float2 t) {
+    const float dx = t.x - 1.0f, dy = t.y - 1.0f;
+    if (fabsf(dx) < 0.5f && fabsf(dy) < 0.5f)
+        return (Acc)__float2int_rn(__fmul_rn(__fadd_rn(dx, dy), kFixScale)) + (2ll << 30);
+    return fix(t.x) + fix(t.y);
 }
 
 // Grid averages <rho>, <rho |u|>, <|Pi|> of the current step before any
 // collision (update_avg_mag, macroscopics.cuh:50-120), for CM_OPT.  The nodes
 // split as in the step kernel.  Units the tiles take (special bit clear; in a
 // neighbour-access step also off the perimeter) load their 18 populations
-// directly and are worked out in packed arithmetic, the two nodes' terms
-// added before their rounding to fixed point; a warp takes 32 units of one
-// row at a time, its next place found without a division.  The parity's
+// directly and are worked out in packed arithmetic, each node's terms rounded
+// to fixed point by themselves; a warp takes 32 units of one row at a time, its next place found without a division.  The parity's
 // general-path units are spread over every thread of the grid, one node each,
 // through the general path.  The terms are summed in exact fixed point, so
 // the averages do not depend on the order.
@@ -883,9 +891,9 @@ __global__ void __launch_bounds__(kPrepassThreads, kPrepassCtas) opt_prepass_ker
         const V2 pxx = (f[1] + f[3]) + d, pyy = (f[2] + f[4]) + d;
         const V2 pxy = (f[5] + f[7]) - (f[6] + f[8]);
         const V2 pi = vsqrt(fma(pxx, pxx, fma(2.0f * pxy, pxy, pyy * pyy)));
-        v[0] += fix_near(rho.v.x + rho.v.y, 2.0f);
-        v[4] += fix_near(jm.v.x + jm.v.y, 0.0f);
-        v[5] += fix_near(pi.v.x + pi.v.y, 0.0f);
+        v[0] += fix_two_densities(rho.v);
+        v[4] += fix_two(jm.v);
+        v[5] += fix_two(pi.v);
     }
     // (from the last thread down: on small lattices the last warps have no units)
     const int nthreads = gridDim.x * kPrepassThreads;

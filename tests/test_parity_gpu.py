@@ -347,3 +347,25 @@ def test_nonfinite_detection():
     with pytest.raises(lbmx.LbmxError) as e:
         L.step(2, flags=lbmx.STEP_STORE_MOMENTS | lbmx.STEP_CHECK_FINITE)
     assert e.value.code == 7
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 17), (130, 33), (66, 3)])
+def test_averages_take_each_density_at_full_precision(nx, ny):
+    """CM_OPT: the pre-pass' mass sum is the sum of every node's density,
+    each rounded to 2^-30 by itself, to the last unit."""
+    c = C.random_state(C.taylor_green(nx, ny, op=C.CM_OPT, nu=0.05), seed=3)
+    L = C.make_lattice(c)
+    f = L.populations()
+    cx, cy = [0, 1, 0, -1, 0, 1, -1, -1, 1], [0, 0, 1, 0, -1, 1, 1, -1, -1]
+    f = [np.roll(f[q], (cy[q], cx[q]), axis=(0, 1)) for q in range(9)]
+    rho = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7])) + f[8]
+    # the perimeter's units of two nodes take the general path, which adds in order
+    edge = np.ones((ny, nx), bool)
+    edge[1:-1, 2:-2] = False
+    seq = f[0]
+    for q in range(1, 9):
+        seq = seq + f[q]
+    rho = np.where(edge, seq, rho)
+    assert rho.dtype == np.float32
+    want = int(np.rint(rho.astype(np.float64) * 2.0 ** 30).astype(np.int64).sum())
+    assert int(L.opt_partials()[0]) == want
