@@ -276,8 +276,6 @@ __device__ __forceinline__ W2& operator-=(W2& a, W2P b) { return a = a - b; }
 // lanes: the nodes of a value (one, or two)
 __device__ __forceinline__ float& lane_of(float& v, int) { return v; }
 __device__ __forceinline__ float& lane_of(W2& v, int h) { return h ? v.v.y : v.v.x; }
-__device__ __forceinline__ float lanes_sum(float v) { return v; }
-__device__ __forceinline__ float lanes_sum(W2 v) { return v.v.x + v.v.y; }
 __device__ __forceinline__ float recip(float v) { return 1.0f / v; }
 __device__ __forceinline__ W2 recip(W2 v) { return W2{make_float2(1.0f / v.v.x, 1.0f / v.v.y)}; }
 template <typename R>
@@ -686,7 +684,8 @@ __device__ __forceinline__ void adj_node_vjp(const AdjArgs& a, const AdjNode* nd
     const R b_ux0 = sc * b_ux, b_uy0 = sc * b_uy;
     b_gm -= 0.5f * sc * R(ux0 * b_ux0 + uy0 * b_uy0);
     // Guo correction: u0 = (j + F0 / 2) / rho
-    const R b_jx = b_ux0 * inv, b_jy = b_uy0 * inv;
+    const R bx = b_ux0 * inv, by = b_uy0 * inv;
+    const R b_jx = R(b_ux0 - bx * rho) * inv + bx, b_jy = R(b_uy0 - by * rho) * inv + by;
     b_fx += 0.5f * b_jx;
     b_fy += 0.5f * b_jy;
     b_rho -= ux0 * b_jx + uy0 * b_jy;
@@ -812,7 +811,7 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjNodes<OP> == 2 ? kAdjReverseBlo
     using R = AdjReal<OP>;
     constexpr int N = kAdjNodes<OP>;
     const long long n = a.g.n;
-    float sums[3] = {0.f, 0.f, 0.f}, omega_low = 0.f, asums[3] = {0.f, 0.f, 0.f};
+    float sums[3] = {0.f, 0.f, 0.f}, low[3] = {0.f, 0.f, 0.f}, asums[3] = {0.f, 0.f, 0.f};
     const uint32_t node0 = blockIdx.x * (N * kAdjBlock) + threadIdx.x;
     if (node0 < n) {
         AdjNode nd[N];
@@ -873,25 +872,28 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjNodes<OP> == 2 ? kAdjReverseBlo
             g_gamma[node] = (OP != LBMX_CM ? gg[h] : g_gamma[node]) + (double)lane_of(d_gamma, h);
         }
         // (the first node's term, then what adding the second's rounded off)
-        sums[0] = lane_of(d_omega, 0);
-        if (N == 2) two_sum(sums[0], omega_low, lane_of(d_omega, N - 1));
-        sums[1] = lanes_sum(d_fx);
-        sums[2] = lanes_sum(d_fy);
+        R d[3] = {d_omega, d_fx, d_fy};
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            sums[k] = lane_of(d[k], 0);
+            if (N == 2) two_sum(sums[k], low[k], lane_of(d[k], N - 1));
+        }
     }
-    // The rate's derivative is a sum of terms of both signs, often far below
-    // their magnitudes: its warp sums keep what the additions round off.
+    // The scalars' derivatives are sums of terms of both signs, often far
+    // below their magnitudes: the warp sums keep what the additions round off.
     __shared__ double sh[kAdjBlock / 32][3];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        const float sb = __shfl_down_sync(0xffffffffu, sums[0], o), eb = __shfl_down_sync(0xffffffffu, omega_low, o);
-        two_sum(sums[0], omega_low, sb);
-        omega_low += eb;
 #pragma unroll
-        for (int k = 1; k < 3; k++) sums[k] += __shfl_down_sync(0xffffffffu, sums[k], o);
+        for (int k = 0; k < 3; k++) {
+            const float sb = __shfl_down_sync(0xffffffffu, sums[k], o), eb = __shfl_down_sync(0xffffffffu, low[k], o);
+            two_sum(sums[k], low[k], sb);
+            low[k] += eb;
+        }
     }
     if (lane == 0)
-        for (int k = 0; k < 3; k++) sh[warp][k] = (double)sums[k] + (k == 0 ? (double)omega_low : 0.0);
+        for (int k = 0; k < 3; k++) sh[warp][k] = (double)sums[k] + (double)low[k];
     __syncthreads();
     if (threadIdx.x < 3) {
         double t = 0.0;
