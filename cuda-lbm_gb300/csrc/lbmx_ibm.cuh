@@ -190,18 +190,6 @@ __device__ void ibm_iterate(const IbmData<R>& a, const IbmSmem<R>& s) {
     else ibm_iterate_s<R, 4>(a, s);
 }
 
-// All rounds of one step with the patch read from a.patch_rho / a.patch_u;
-// sm holds ibm_smem_bytes_of<R> bytes.
-template <typename R>
-__device__ void ibm_rounds(const IbmData<R>& a, R* sm) {
-    const IbmSmem<R> s = ibm_layout(a, sm);
-    ibm_stage(a, s);
-    for (int i = threadIdx.x; i < a.npatch; i += blockDim.x)
-        ibm_set_patch(s, i, a.patch_rho[i], a.patch_u[i], a.patch_u[a.npatch + i]);
-    __syncthreads();
-    ibm_iterate(a, s);
-}
-
 // ---------------------------------------------------------------------------
 // The engine's (float) form of the same rounds, laid out for few shared-
 // memory transactions: a patch node's working velocity, density and

@@ -202,8 +202,6 @@ struct IbmData {
     const float* sten_w;                // [nm][stencil^2] kernel weight
     const int* spread;                  // [npatch + 1] offsets, then the stencil points of each patch node (ascending)
     const int* patch_nodes;             // [npatch] node offset (y*pitch + x)
-    const R* patch_rho;                 // [npatch]
-    const R* patch_u;                   // [2][npatch] uncorrected velocity
     R* marker_u;                        // [2][nm] last interpolated velocity
     R* marker_rho;                      // [nm]
     R* marker_force;                    // [2][nm] summed over iterations
