@@ -1316,18 +1316,21 @@ lbmx_status lbmx_adjoint_forward(lbmx_adjoint* a, int32_t nsteps, double* object
     if (!a->have_state) return afail(a, LBMX_ERR_NOT_INITIALIZED, "lbmx_adjoint_forward: call lbmx_adjoint_set_state first");
     if (nsteps < 1) return afail(a, LBMX_ERR_INVALID_ARGUMENT, "lbmx_adjoint_forward: nsteps < 1");
     cudaSetDevice(a->p.device);
+    a->have_forward = false;
     const size_t state = (size_t)9 * a->n;
     // checkpoints: the states at t = 0 (pc0 itself), every, 2 every, ...
     const int ncheck = (nsteps + a->every - 1) / a->every;
     if (ncheck > a->ncheck_cap) {
         cudaFree(a->ckpt);
         a->ckpt = nullptr;
+        a->ncheck_cap = 0;
         if (ncheck > 1) ADJ_CUDA(a, device_alloc(&a->ckpt, (size_t)(ncheck - 1) * state * sizeof(float)));
         a->ncheck_cap = ncheck;
     }
     if (nsteps + 1 > a->avg_cap) {
         cudaFree(a->avg_hist);
         a->avg_hist = nullptr;
+        a->avg_cap = 0;
         ADJ_CUDA(a, device_alloc(&a->avg_hist, (size_t)3 * (nsteps + 1) * sizeof(float)));
         a->avg_cap = nsteps + 1;
     }

@@ -67,6 +67,7 @@ cudaError_t lbmx::device_alloc(void** p, size_t bytes) {
         s->busy = false;
         if (freed && (e = cudaMalloc(p, bytes)) != cudaErrorMemoryAllocation) return e;
     }
+    cudaGetLastError();  // the caller has it; the next launch's check is not to find it
     return e;
 }
 

@@ -511,6 +511,7 @@ lbmx_status lbmx_tangent_run(lbmx_tangent* t, int32_t nsteps, double* series) {
     if (series && nsteps > t->series_cap) {
         cudaFree(t->series);
         t->series = nullptr;
+        t->series_cap = 0;
         TAN_CUDA(t, device_alloc(&t->series, (size_t)4 * nsteps * sizeof(double)));
         t->series_cap = nsteps;
     }

@@ -172,6 +172,32 @@ def test_backward_twice_after_one_forward(op, steps, every):
     assert s2 == s
 
 
+def test_a_forward_run_without_room_leaves_nothing_to_go_back_over():
+    torch = pytest.importorskip("torch")
+    n = 1024  # 36 MB a state
+    a = lbmx.Adjoint(n, n, op=C.BGK, omega=1.2, periodic=(True, True), checkpoint_every=1)
+    a.set_state(np.ones((n, n), np.float32), np.zeros((2, n, n), np.float32))
+    w = np.zeros((3, n, n), np.float32)
+    w[1] = 1.0
+    a.set_objective(w, 1)
+    a.forward(3)
+    a.backward()
+    torch.cuda.empty_cache()
+    full = torch.empty(torch.cuda.mem_get_info()[0] - (512 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(lbmx.LbmxError) as e:
+            a.forward(40)
+        assert e.value.code == 2
+        with pytest.raises(lbmx.LbmxError) as e:
+            a.backward()
+        assert e.value.code == 5
+        a.forward(3)
+        a.backward()
+    finally:
+        del full
+        torch.cuda.empty_cache()
+
+
 def test_autograd_retained_graph_gives_the_same_gradient_again():
     torch = pytest.importorskip("torch")
     import lbmx_autograd
