@@ -779,12 +779,13 @@ __global__ void adj_forward_kernel(const AdjArgs a, const float* pc_prev, float*
     if (objective && a.weights) {
         const float w0 = a.weights[node], w1 = (a.weights + n)[node], w2 = (a.weights + 2 * n)[node];
         const float mx = mom[0] * mom[1], my = mom[0] * mom[2];
-        // a node without weight adds nothing (unless its moments are not
-        // finite): no FP64 arithmetic, on a pipe that was two thirds busy
-        // with it, and no read and write of its 8-byte sum
-        if (w0 != 0.0f || w1 != 0.0f || w2 != 0.0f || !isfinite(mom[0] + mx + my)) {
+        const float scale = !a.drag ? 1.0f : a.gamma ? a.gamma[node] : 0.0f;
+        // a node without weight adds nothing (unless its moments or its
+        // factor are not finite): no FP64 arithmetic, on a pipe that was two
+        // thirds busy with it, and no read and write of its 8-byte sum
+        if (w0 != 0.0f || w1 != 0.0f || w2 != 0.0f || !isfinite(mom[0] + mx + my) || !isfinite(scale)) {
             const double term = (double)w0 * mom[0] + (double)w1 * mx + (double)w2 * my;
-            jnode[node] += a.drag ? (double)(a.gamma ? a.gamma[node] : 0.0f) * term : term;
+            jnode[node] += a.drag ? (double)scale * term : term;
         }
     }
     if (rho_out) {
@@ -893,7 +894,8 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjNodes<OP> == 2 ? kAdjReverseBlo
         }
     }
     if (lane == 0)
-        for (int k = 0; k < 3; k++) sh[warp][k] = (double)sums[k] + (double)low[k];
+        // (beside a sum that is not finite there is nothing to keep)
+        for (int k = 0; k < 3; k++) sh[warp][k] = (double)sums[k] + (isfinite(low[k]) ? (double)low[k] : 0.0);
     __syncthreads();
     if (threadIdx.x < 3) {
         double t = 0.0;

@@ -198,6 +198,22 @@ def test_a_forward_run_without_room_leaves_nothing_to_go_back_over():
         torch.cuda.empty_cache()
 
 
+@pytest.mark.parametrize("op", [C.BGK, C.MRT, C.CM, C.CM_OPT])
+def test_overflow_is_infinite_and_an_infinite_factor_is_seen(op):
+    c = case(op, gamma_scale=0.0)
+    a = make_adjoint(c)
+    w = np.zeros((3, NY, NX), np.float32)
+    w[1] = 3e38
+    a.set_objective(w, 1)
+    a.forward(1)
+    assert a.backward()[1][1] == np.inf  # 0.5 / rho of it for every node: a sum beyond FP32
+    g = np.zeros((NY, NX), np.float32)
+    g[3, 4] = np.inf
+    a.set_gamma(g)
+    a.set_objective(np.zeros((3, NY, NX), np.float32), 1, kind=lbmx.OBJECTIVE_BRINKMAN_DRAG)
+    assert np.isnan(a.forward(1))  # infinity times a weightless node's zero
+
+
 def test_autograd_retained_graph_gives_the_same_gradient_again():
     torch = pytest.importorskip("torch")
     import lbmx_autograd
