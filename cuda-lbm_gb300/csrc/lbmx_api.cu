@@ -466,7 +466,7 @@ struct ReadbackArgs {
     float* u;
     const double* sums;
     const unsigned int* error_word;
-    double* mail;      // [4] sums 0..2, then the error word
+    double* mail;      // [5] sums 0..2, the error word; lbmx_synchronize's copy of that
 };
 constexpr int kReadbackRows = 8;
 __global__ void __launch_bounds__(32 * kReadbackRows) readback_kernel(const ReadbackArgs a, int vec) {
@@ -686,7 +686,7 @@ lbmx_status lbmx_create(const lbmx_params* p, lbmx_handle** out) {
     // work counters, the averages, the last-block counter and the error word
     const size_t words = (size_t)(kAccSets * kAccPerSet + kSumsBufferLen + 4) * 8 + 5 * 4;
     ALLOC(h->words, words);
-    if (cudaMallocHost((void**)&h->mail, 4 * sizeof(double)) != cudaSuccess) {
+    if (cudaMallocHost((void**)&h->mail, 5 * sizeof(double)) != cudaSuccess) {
         fail(nullptr, LBMX_ERR_OUT_OF_MEMORY, "lbmx_create: cudaMallocHost failed");
         lbmx_destroy(h);
         return LBMX_ERR_OUT_OF_MEMORY;
@@ -1701,7 +1701,7 @@ lbmx_status lbmx_write_vti(lbmx_handle* h, const char* path) {
 lbmx_status lbmx_synchronize(lbmx_handle* h) {
     if (!h) return fail(h, LBMX_ERR_INVALID_ARGUMENT, "lbmx_synchronize: NULL handle");
     cudaSetDevice(h->p.device);
-    unsigned int* w = reinterpret_cast<unsigned int*>(h->mail);
+    unsigned int* w = reinterpret_cast<unsigned int*>(h->mail + 4);  // its own word: another thread may be reading moments
     LBMX_CUDA(h, cudaMemcpyAsync(w, h->error_word, sizeof(*w), cudaMemcpyDeviceToHost, h->stream));
     LBMX_CUDA(h, cudaStreamSynchronize(h->stream));
     return check_word(h, *w);

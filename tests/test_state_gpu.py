@@ -272,3 +272,26 @@ def test_moments_into_device_fields_at_any_address(nx, offset):
     np.testing.assert_array_equal(got[:n].reshape(ny, nx), rho)
     np.testing.assert_array_equal(got[n:].reshape(2, ny, nx), u)
     assert list(s) == list(sums)
+
+
+def test_synchronize_while_another_thread_reads_the_moments():
+    import threading
+    L = C.make_lattice(C.random_state(C.cavity_moving_wall(64, 48, op=C.BGK), seed=3))
+    L.step(3)
+    want = list(L.moments()[2])
+    done = threading.Event()
+
+    def wait():
+        while not done.is_set():
+            L.synchronize()
+
+    t = threading.Thread(target=wait)
+    t.start()
+    try:
+        s = (ctypes.c_double * 3)()
+        for _ in range(5000):
+            L._check(L.lib.lbmx_moments(L.h, None, None, s))
+            assert list(s) == want
+    finally:
+        done.set()
+        t.join()
