@@ -802,12 +802,13 @@ __device__ __forceinline__ void opt_terms(const StepArgs& a, long long off, cons
 }
 
 // fix() of two nodes' terms, each rounded alone, by 32-bit conversions of
-// their products with 2^30 while both are below one, fix() itself otherwise
-// (NaN included).
+// their products with 2^30 while both are below one, fix() itself otherwise.
+// (Two NaN, each of which converts to -2^63, add up to zero: the nodes of a
+// diverged lattice go without conversions on the FP64 pipe.)
 __device__ __forceinline__ Acc fix_two(float2 t) {
     if (fabsf(t.x) < 1.0f && fabsf(t.y) < 1.0f)
         return (Acc)(__float2int_rn(__fmul_rn(t.x, kFixScale)) + __float2int_rn(__fmul_rn(t.y, kFixScale)));
-    return fix(t.x) + fix(t.y);
+    return isnan(t.x) && isnan(t.y) ? 0 : fix(t.x) + fix(t.y);
 }
 // The same for two densities, with one conversion: above 1/2 and below 3/2
 // their differences from 1 are multiples of 2^-24, and so is the differences'
@@ -816,7 +817,7 @@ __device__ __forceinline__ Acc fix_two_densities(float2 t) {
     const float dx = t.x - 1.0f, dy = t.y - 1.0f;
     if (fabsf(dx) < 0.5f && fabsf(dy) < 0.5f)
         return (Acc)__float2int_rn(__fmul_rn(__fadd_rn(dx, dy), kFixScale)) + (2ll << 30);
-    return fix(t.x) + fix(t.y);
+    return isnan(t.x) && isnan(t.y) ? 0 : fix(t.x) + fix(t.y);
 }
 
 // Grid averages <rho>, <rho |u|>, <|Pi|> of the current step before any
