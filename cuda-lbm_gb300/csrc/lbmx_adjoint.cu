@@ -39,12 +39,15 @@ namespace {
 
 // Threads per block of every adjoint kernel, and resident blocks per SM the
 // reverse kernel's registers are bounded for.  Neither kernel reaches memory
-// speed: 2048 x 1024 CM, reverse 95 us for 285 MB (a floor of 42 us at the
-// measured copy rate; latency of its 20 loads a node with 16 warps an SM, two
-// nodes a thread in packed arithmetic: five blocks spill, three are 112 us;
-// one node a thread 107 us), forward 37 us (floor 22 to 31, instruction
-// issue).  With a 64-bit division for the coordinates, wrap tests on every
-// link and FP64 objective terms on every node they took 149 and 51 us.
+// speed: 2048 x 1024 CM, reverse 96 us for 285 MB (a floor of 42 us at the
+// measured copy rate), forward 37 us (floor 22 to 31, instruction issue).  The
+// reverse is one dependent chain a node pair -- loads, moments, adjoints --
+// with 16 warps an SM to hide it behind: 42 % of issue slots, waits on loads
+// 30 % and on fixed-latency arithmetic 20 % of a warp's time; loads two chunks
+// ahead changed nothing.  (Two nodes a thread in packed arithmetic: five
+// blocks spill, three are 112 us; one node a thread 107 us.)  With a 64-bit
+// division for the coordinates, wrap tests on every link and FP64 objective
+// terms on every node they took 149 and 51 us.
 constexpr int kAdjBlock = 128;
 constexpr int kAdjReverseBlocks1 = 5, kAdjReverseBlocks2 = 4;  // one and two nodes a thread
 constexpr int kTan = 2;  // tangents per pass
@@ -276,6 +279,8 @@ __device__ __forceinline__ W2& operator-=(W2& a, W2P b) { return a = a - b; }
 // lanes: the nodes of a value (one, or two)
 __device__ __forceinline__ float& lane_of(float& v, int) { return v; }
 __device__ __forceinline__ float& lane_of(W2& v, int h) { return h ? v.v.y : v.v.x; }
+__device__ __forceinline__ float lanes_down(float v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ W2 lanes_down(W2 v, int o) { return W2{make_float2(lanes_down(v.v.x, o), lanes_down(v.v.y, o))}; }
 __device__ __forceinline__ float recip(float v) { return 1.0f / v; }
 __device__ __forceinline__ W2 recip(W2 v) { return W2{make_float2(1.0f / v.v.x, 1.0f / v.v.y)}; }
 template <typename R>
@@ -812,7 +817,8 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjNodes<OP> == 2 ? kAdjReverseBlo
     using R = AdjReal<OP>;
     constexpr int N = kAdjNodes<OP>;
     const long long n = a.g.n;
-    float sums[3] = {0.f, 0.f, 0.f}, low[3] = {0.f, 0.f, 0.f}, asums[3] = {0.f, 0.f, 0.f};
+    float omega = 0.f, omega_low = 0.f, asums[3] = {0.f, 0.f, 0.f};
+    R force[2] = {};
     const uint32_t node0 = blockIdx.x * (N * kAdjBlock) + threadIdx.x;
     if (node0 < n) {
         AdjNode nd[N];
@@ -873,29 +879,33 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjNodes<OP> == 2 ? kAdjReverseBlo
             g_gamma[node] = (OP != LBMX_CM ? gg[h] : g_gamma[node]) + (double)lane_of(d_gamma, h);
         }
         // (the first node's term, then what adding the second's rounded off)
-        R d[3] = {d_omega, d_fx, d_fy};
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            sums[k] = lane_of(d[k], 0);
-            if (N == 2) two_sum(sums[k], low[k], lane_of(d[k], N - 1));
-        }
+        omega = lane_of(d_omega, 0);
+        if (N == 2) two_sum(omega, omega_low, lane_of(d_omega, N - 1));
+        force[0] = d_fx;
+        force[1] = d_fy;
     }
-    // The scalars' derivatives are sums of terms of both signs, often far
-    // below their magnitudes: the warp sums keep what the additions round off.
+    // The rate's derivative is a sum of terms of both signs, often far below
+    // their magnitudes: its warp sums keep what the additions round off.  The
+    // force's are FP32 sums over 32 nodes, one a lane of the packed pair.
     __shared__ double sh[kAdjBlock / 32][3];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
+        const float sb = __shfl_down_sync(0xffffffffu, omega, o), eb = __shfl_down_sync(0xffffffffu, omega_low, o);
+        two_sum(omega, omega_low, sb);
+        omega_low += eb;
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const float sb = __shfl_down_sync(0xffffffffu, sums[k], o), eb = __shfl_down_sync(0xffffffffu, low[k], o);
-            two_sum(sums[k], low[k], sb);
-            low[k] += eb;
+        for (int k = 0; k < 2; k++) force[k] = force[k] + lanes_down(force[k], o);
+    }
+    if (lane == 0) {
+        // (beside a sum that is not finite there is nothing to keep)
+        sh[warp][0] = (double)omega + (isfinite(omega_low) ? (double)omega_low : 0.0);
+        for (int k = 0; k < 2; k++) {
+            double t = (double)lane_of(force[k], 0);
+            if (N == 2) t += (double)lane_of(force[k], N - 1);
+            sh[warp][1 + k] = t;
         }
     }
-    if (lane == 0)
-        // (beside a sum that is not finite there is nothing to keep)
-        for (int k = 0; k < 3; k++) sh[warp][k] = (double)sums[k] + (isfinite(low[k]) ? (double)low[k] : 0.0);
     __syncthreads();
     if (threadIdx.x < 3) {
         double t = 0.0;
