@@ -39,11 +39,11 @@ namespace {
 
 // Threads per block of every adjoint kernel, and resident blocks per SM the
 // reverse kernel's registers are bounded for.  Neither kernel reaches memory
-// speed: 2048 x 1024 CM, reverse 96 us for 285 MB (a floor of 42 us at the
+// speed: 2048 x 1024 CM, reverse 94 us for 285 MB (a floor of 42 us at the
 // measured copy rate), forward 37 us (floor 22 to 31, instruction issue).  The
 // reverse is one dependent chain a node pair -- loads, moments, adjoints --
-// with 16 warps an SM to hide it behind: 42 % of issue slots, waits on loads
-// 30 % and on fixed-latency arithmetic 20 % of a warp's time; loads two chunks
+// with 16 warps an SM to hide it behind: 40 % of issue slots, waits on loads
+// 31 % and on fixed-latency arithmetic 21 % of a warp's time; loads two chunks
 // ahead changed nothing.  (Two nodes a thread in packed arithmetic: five
 // blocks spill, three are 112 us; one node a thread 107 us.)  With a 64-bit
 // division for the coordinates, wrap tests on every link and FP64 objective

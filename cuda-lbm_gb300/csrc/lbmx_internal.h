@@ -320,9 +320,9 @@ __host__ __device__ constexpr int step_tile_h(int elem_bytes) { return elem_byte
 // least (64 x 12: 1.24 nodes of the first step per node, 32 x 8: 1.41 with
 // units of two) -- as long as three CTAs of two stages each fit an SM's
 // shared memory, since the collision's chain of dependent arithmetic wants
-// warps: an 8192^2 FP32 cavity takes 402 us a step with 64 x 12 and three
-// CTAs, 427 with 64 x 16 and two, 460 with 64 x 12 and two, 492 with 64 x 8
-// and four; FP16 391 with 64 x 20, 416 with 64 x 16 (single steps: 740 and
+// warps: an 8192^2 FP32 cavity takes 397 us a step with 64 x 12 and three
+// CTAs (402 when the shapes were compared: 427 with 64 x 16 and two, 460 with
+// 64 x 12 and two, 492 with 64 x 8 and four); FP16 391 with 64 x 20, 416 with 64 x 16 (single steps: 740 and
 // 414).  CM needs more than the 72 registers a thread has with three CTAs:
 // FP32 CM takes 64 x 16 and two (4096^2: 133.5 us, 134.9 with 64 x 12 and
 // three; 1024^2: 10.6 and 11.3).

@@ -833,7 +833,9 @@ __device__ __forceinline__ Acc fix_two_densities(float2 t) {
 // Instruction issue bounds it (three roots and divisions a node): node by
 // node, with 64-bit addresses, 220 instructions a node took 48.6 us for
 // 4096 x 1024 (151 MB, 22 us at the measured copy rate), 31 to 32 now.
-constexpr int kPrepassThreads = 256, kPrepassCtas = 4;  // (three CTAs per SM: 89 us a step, five spill: 90; four 85)
+// CTAs per SM: four (the step 85 us when they were compared, three 89, five
+// spill: 90; 86.4 since each node's terms are rounded by themselves)
+constexpr int kPrepassThreads = 256, kPrepassCtas = 4;
 template <typename T, int P>
 __global__ void __launch_bounds__(kPrepassThreads, kPrepassCtas) opt_prepass_kernel(const StepArgs a) {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -19,8 +19,8 @@
 //
 // Single steps of a large FP32 lattice are bound by HBM (72 bytes a node and
 // step, issue slots a third busy); a pair moves the same bytes for two steps
-// and is bound by issue and latency instead: MRT cavity 8192^2 740 -> 402 us
-// a step (90.7 -> 167 GLUPS), 1024^2, in L2, 12.1 -> 8.6 us, 256^2 vortex 4.3
+// and is bound by issue and latency instead: MRT cavity 8192^2 740 -> 397 us
+// a step (90.7 -> 169 GLUPS), 1024^2, in L2, 12.1 -> 8.4 us, 256^2 vortex 4.3
 // -> 2.6 us (half the launches), FP16 8192^2 414 -> 391 us (issue-bound both
 // ways).  Tile shapes and their choice: pair_shape in lbmx_internal.h.
 #pragma once
@@ -66,7 +66,7 @@ __device__ __forceinline__ constexpr int pair_own(int p, int dx, int dy) {
 // of 2^30, a unit's mass less the 2 it has at rest -- and a warp adds its
 // total to its own 64-bit accumulators in shared memory when one of its
 // threads' sums passes kUnitSumLimit at the end of a tile (at most three
-// units more fit then), and at the end.  Terms out of that range go to the
+// units more fit then), and at the end, the rest mass by the count of units.  Terms out of that range go to the
 // warp's accumulators by themselves.  (64-bit accumulators of both steps in
 // every thread cost 12 registers and twice the instructions; a warp's total
 // after every tile and step: 1024^2 FP32 with sums 10.2 us a step, 9.9 now,
